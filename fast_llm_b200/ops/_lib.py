@@ -128,7 +128,18 @@ def check(status: int, what: str) -> None:
 
 
 def stream_ptr() -> int:
-    return torch.cuda.current_stream().cuda_stream
+    # The raw handle straight from the C binding: `torch.cuda.current_stream()` builds a Stream object after a walk through
+    # Python device helpers, 10 us per call on the host of a B200 box (this: 0.2 us), and every kernel launch asks for it.
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
+
+
+class KernelFunction(torch.autograd.Function):
+    """`autograd.Function` for the hand-written nodes.  The stock `apply` inspects the arguments for functorch wrappers in Python
+    (about 5 us per node); these nodes call raw kernels and cannot run under functorch transforms anyway."""
+
+    @classmethod
+    def apply(cls, *args):
+        return super(torch.autograd.Function, cls).apply(*args)
 
 
 def ptr(t: "torch.Tensor | None") -> int | None:

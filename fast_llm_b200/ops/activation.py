@@ -9,6 +9,7 @@ import enum
 import torch
 
 from fast_llm_b200.ops import _lib
+from fast_llm_b200.ops._lib import KernelFunction
 
 
 class ActivationType(str, enum.Enum):
@@ -83,7 +84,7 @@ def act_bwd_native(grad_out2, x2, gated: bool, act: ActivationType, recompute: b
     return grad_in, out
 
 
-class _MLPActivation(torch.autograd.Function):
+class _MLPActivation(KernelFunction):
     @staticmethod
     def forward(ctx, x, gated, act):
         shape = x.shape

@@ -12,6 +12,7 @@ epilogue straight into the parameter's gradient buffer.  Parity: `fast_llm/funct
 
 import torch
 
+from fast_llm_b200.ops._lib import KernelFunction
 from fast_llm_b200.ops.gemm import matmul_nn, matmul_nt, matmul_tn
 from fast_llm_b200.ops.param_grad import accumulate_param_grad, wgrad_target
 from fast_llm_b200.parallel import fused_tp
@@ -40,7 +41,7 @@ def bias_grad(dy2: torch.Tensor, bias: torch.Tensor):
     return accumulate_param_grad(bias, dy2.sum(0, dtype=torch.float32).to(bias.dtype) if dy2.dtype != torch.float32 else dy2.sum(0))
 
 
-class _Linear(torch.autograd.Function):
+class _Linear(KernelFunction):
     @staticmethod
     def forward(ctx, x, weight, bias, transposed_weight, mode, group, sequence_parallel):
         shape = x.shape

@@ -15,6 +15,7 @@ import enum
 
 import torch
 
+from fast_llm_b200.ops._lib import KernelFunction
 from fast_llm_b200.ops.activation import ActivationType, _native as _act_native, act_bwd_native, act_fwd_native, mlp_activation_reference
 from fast_llm_b200.ops.gemm import gated_ok, matmul_nn, matmul_nt, matmul_nt_gated
 from fast_llm_b200.ops.linear import bias_grad, weight_grad
@@ -57,7 +58,7 @@ def _act_bwd(da, h, gated, act, recompute):
     return dh, (a.detach() if recompute else None)
 
 
-class _MLP(torch.autograd.Function):
+class _MLP(KernelFunction):
     @staticmethod
     def forward(ctx, x, w1, b1, w2, b2, gated, act, group, sequence_parallel, recompute):
         shape = x.shape

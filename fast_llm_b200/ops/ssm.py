@@ -17,6 +17,8 @@ import typing
 
 import torch
 
+from fast_llm_b200.ops._lib import KernelFunction
+
 
 # ----------------------------------------------------------------------------------------------------------------------
 # chunk loop with boundary-state checkpointing
@@ -120,7 +122,7 @@ def causal_conv1d_reference(x, weight, bias, document_index, activation) -> torc
     return activation_reference(out, activation).to(x.dtype)
 
 
-class _CausalConv1d(torch.autograd.Function):
+class _CausalConv1d(KernelFunction):
     TOKENS_PER_BLOCK = 64
 
     @staticmethod
@@ -200,7 +202,7 @@ def _selective_scan_step(state, chunk_in, shared):
     return y.to(x.dtype), states[-1]
 
 
-class _SelectiveScan(torch.autograd.Function):
+class _SelectiveScan(KernelFunction):
     """Chunk-parallel CUDA scan (`csrc/ssm.cu`): three launches forward, four backward; the only saved state beyond the
     inputs is the [chunks, state, channels] start state and decay product of every 64-token chunk."""
 
@@ -337,7 +339,7 @@ def _chunk_layout(boundaries: list[int], chunk: int, device):
     return index.to(device), first
 
 
-class _DeltaStateScan(torch.autograd.Function):
+class _DeltaStateScan(KernelFunction):
     """State entering every chunk of S_{c+1} = decay_c o S_c - mix_c S_c + write_c (zero at document starts): one CUDA kernel
     walks the chunks (`flb_delta_state_scan`), a second one the adjoint recurrence; the gradients of mix, write and decay are
     batched products of the two results."""

@@ -18,7 +18,7 @@ import torch
 from fast_llm_b200.ops._lib import KernelFunction
 from fast_llm_b200.ops.activation import ActivationType, _native as _act_native, act_bwd_native, act_fwd_native, mlp_activation_reference
 from fast_llm_b200.ops.gemm import gated_ok, matmul_nn, matmul_nt, matmul_nt_gated
-from fast_llm_b200.ops.linear import bias_grad, weight_grad
+from fast_llm_b200.ops.linear import bias_grad, needs_weight_grad, weight_grad
 from fast_llm_b200.parallel import fused_tp
 from fast_llm_b200.parallel.ops import gather_op, reduce_op, reduce_scatter_op
 
@@ -118,7 +118,7 @@ class _MLP(KernelFunction):
             if b1 is not None:
                 h = h + b1
         da = matmul_nt(dy2, w2)  # [tokens, ffn] = dy @ W2^T with W2 stored [ffn, hidden]
-        dh, a_re = _act_bwd(da, h, gated, act, a is None)
+        dh, a_re = _act_bwd(da, h, gated, act, a is None and needs_weight_grad(w2))
         a = a_re if a is None else a
         dw2 = weight_grad(dy2, a, w2, transposed_weight=True)
         del a, da
@@ -159,7 +159,7 @@ def _backward_fused(ctx, dy2, x_saved, h, a):
     da = fused.matmul_gathered(pending_dy, w2, False)  # [tokens, ffn/tp] = gather(dy) @ W2^T
     if h is None:
         h = fused.matmul_gathered(pending_x, w1, False)
-    dh, a_re = _act_bwd(da, h, gated, act, a is None)
+    dh, a_re = _act_bwd(da, h, gated, act, a is None and needs_weight_grad(w2))
     a = a_re if a is None else a
     del da
     dy_full = fused.finish_gather(pending_dy)

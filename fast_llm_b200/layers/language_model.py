@@ -357,7 +357,10 @@ class LanguageModelHead(Layer):
     def _logits_only(self, hidden, kwargs):
         group = self._logits_group
         x = gather_op(hidden, group, 0) if (self._sequence_parallel_logits_gather and group is not None) else hidden
-        logits = matmul_nt(x.detach(), self.output_weights.detach()).float() * self._config.logits_scale_factor
+        # fp32 straight from the accumulators: no bf16 copy to convert afterwards (three passes over [tokens, vocabulary])
+        logits = matmul_nt(x.detach(), self.output_weights.detach(), out_dtype=torch.float32)
+        if self._config.logits_scale_factor != 1.0:
+            logits = logits * self._config.logits_scale_factor
         if self._config.final_logit_softcap is not None:
             cap = self._config.final_logit_softcap
             logits = torch.tanh(logits / cap) * cap

@@ -235,7 +235,6 @@ class GatedDeltaNet(_SSMBase):
         value_head_dim = TensorDim("gdn_value_head_dim", c.value_head_dim)
         key_head_dim = TensorDim("gdn_key_head_dim", c.key_head_dim)
         self._value_heads, self._key_heads = value_heads_dim.size, key_heads_dim.size
-        self._heads_per_key = div(self._value_heads, self._key_heads)
         query_dim = CompositeTensorDim("gdn_query", (key_heads_dim, key_head_dim))
         key_dim = CompositeTensorDim("gdn_key", (key_heads_dim, key_head_dim))
         value_dim = CompositeTensorDim("gdn_value", (value_heads_dim, value_head_dim))
@@ -268,9 +267,6 @@ class GatedDeltaNet(_SSMBase):
         q = q.reshape(tokens, self._key_heads, c.key_head_dim)
         k = k.reshape(tokens, self._key_heads, c.key_head_dim)
         v = v.reshape(tokens, self._value_heads, c.value_head_dim)
-        if self._heads_per_key > 1:
-            q = q.repeat_interleave(self._heads_per_key, dim=1)
-            k = k.repeat_interleave(self._heads_per_key, dim=1)
         beta, alpha = torch.split(ba, [self._value_heads, self._value_heads], dim=-1)
         out = chunk_delta_rule(q, k, v, gdn_log_decay(alpha, self.A_log, self.dt_bias), beta.float().sigmoid(), cu, normalize_qk=True)
         out = self.norm(out.to(x.dtype), z.reshape(tokens, self._value_heads, c.value_head_dim))

@@ -22,6 +22,10 @@ _SIGNATURES = {
     "flb_causal_conv1d_fwd": [_p, _p, _p, _p, _p, _ll, _i, _i, _i, _p],
     "flb_causal_conv1d_bwd": [_p, _p, _p, _p, _p, _p, _p, _p, _ll, _i, _i, _i, _i, _p],
     "flb_delta_state_scan": [_p, _p, _p, _p, _p, _i, _i, _i, _i, _i, _i, _p],
+    "flb_delta_max_chunks": [_ll, _i],
+    "flb_delta_chunks": [_p, _i, _i, _p, _p, _p],
+    "flb_delta_fwd": [_p] * 3 + [_ll] * 3 + [_p] * 2 + [_i] * 6 + [_f] + [_p] * 2 + [_i] * 2 + [_p] * 13,
+    "flb_delta_bwd": [_p] * 2 + [_ll] * 2 + [_p] + [_i] * 6 + [_f] + [_p] * 2 + [_i] * 2 + [_p] * 20,
     "flb_selective_scan_chunks": [_ll],
     "flb_selective_scan_fwd": [_p] * 9 + [_ll, _i, _i, _i, _i, _p, _p, _p, _p],
     "flb_selective_scan_checkpoints": [_ll, _i],

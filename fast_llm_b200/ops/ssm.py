@@ -447,8 +447,89 @@ def _delta_rule_all_chunks(q, k, v, g, beta, boundaries: list[int], chunk: int) 
     return out.transpose(1, 2)[valid].to(out_dtype)
 
 
+class _DeltaRule(KernelFunction):
+    """The delta rule in five kernels (`csrc/delta.cu`): per chunk of 64 tokens the triangular system and its inverse, a scan over
+    the chunks of every document for the states, the outputs; backward, the adjoint scan and the gradients chunk by chunk.
+    q, k may have fewer heads than v (each serves that many adjacent value heads) and any row stride."""
+
+    @staticmethod
+    def applies(q, k, v, g, beta) -> bool:
+        def rows_ok(t):
+            return t.dtype == torch.bfloat16 and t.stride(2) == 1 and t.stride(1) == t.shape[2] and t.stride(0) % 8 == 0 and t.data_ptr() % 16 == 0
+
+        return (q.is_cuda and all(rows_ok(t) for t in (q, k, v)) and g.dtype == torch.float32 and beta.dtype == torch.float32
+                and q.shape[2] in (64, 128) and v.shape[2] in (64, 128) and v.shape[1] % q.shape[1] == 0 and q.shape[0] > 0)
+
+    @staticmethod
+    def forward(ctx, q, k, v, g, beta, cu_seqlens, normalize, scale):
+        from fast_llm_b200.ops import _lib
+
+        lib = _lib.get_lib()
+        g, beta = g.contiguous(), beta.contiguous()
+        tokens, key_heads, dk = q.shape
+        heads, dv = v.shape[1:]
+        repeat, channel = heads // key_heads, g.dim() == 3
+        device = q.device
+        cu = None if cu_seqlens is None else cu_seqlens.to(device=device, dtype=torch.int32)
+        docs = 1 if cu is None else cu.numel()  # with a list: its documents and the padding behind the last one
+        chunks = lib.flb_delta_max_chunks(tokens, docs)
+        need_grad = any(ctx.needs_input_grad[:5])
+
+        def empty(*shape, dtype=torch.float32):
+            return torch.empty(*shape, dtype=dtype, device=device)
+
+        chunk, doc_chunk = empty(chunks, 2, dtype=torch.int32), empty(docs + 1, dtype=torch.int32)
+        _lib.check(lib.flb_delta_chunks(_lib.ptr(cu), docs, tokens, chunk.data_ptr(), doc_chunk.data_ptr(), _lib.stream_ptr()), "flb_delta_chunks")
+        decay = empty(chunks, heads, 64, dk) if channel else empty(chunks, heads, 64)
+        norm_q, norm_k = empty(chunks, heads, 64), empty(chunks, heads, 64)
+        tri_t, tri_p = (empty(chunks, heads, 3, 64, 64, dtype=torch.bfloat16) for _ in range(2))
+        tri_n = empty(chunks, heads, 64, 64) if need_grad else None
+        planes = [empty(chunks, heads, 3, 64, dk, dtype=torch.bfloat16) if channel else None for _ in range(3)]  # k in, k out, q in
+        u, state = empty(chunks, heads, 64, dv), empty(chunks, heads, dv, dk)
+        out = empty(tokens, heads, dv, dtype=torch.bfloat16)
+        _lib.check(lib.flb_delta_fwd(
+            q.data_ptr(), k.data_ptr(), v.data_ptr(), q.stride(0), k.stride(0), v.stride(0), g.data_ptr(), beta.data_ptr(), heads, repeat, dk, dv,
+            int(channel), int(normalize), scale, chunk.data_ptr(), doc_chunk.data_ptr(), docs, chunks, decay.data_ptr(), norm_q.data_ptr(), norm_k.data_ptr(),
+            tri_t.data_ptr(), tri_p.data_ptr(), _lib.ptr(tri_n), *(_lib.ptr(t) for t in planes), u.data_ptr(), state.data_ptr(), out.data_ptr(),
+            _lib.stream_ptr()), "flb_delta_fwd")
+        _lib.count_launch(4)
+        if need_grad:
+            ctx.save_for_backward(q, k, beta, chunk, doc_chunk, decay, norm_q, norm_k, tri_t, tri_p, tri_n, *planes, u, state)
+            ctx.args = (repeat, channel, normalize, scale, docs, g.shape)
+        return out
+
+    @staticmethod
+    def backward(ctx, dout):
+        from fast_llm_b200.ops import _lib
+
+        q, k, beta, chunk, doc_chunk, decay, norm_q, norm_k, tri_t, tri_p, tri_n, k_in, k_out, q_in, u, state = ctx.saved_tensors
+        repeat, channel, normalize, scale, docs, g_shape = ctx.args
+        tokens, key_heads, dk = q.shape
+        chunks, heads, dv = state.shape[:3]
+        dout = dout.to(torch.bfloat16).contiguous()
+        dr, dstate = torch.empty_like(u), torch.empty_like(state)
+        dq, dkey = (torch.empty(tokens, heads, dk, dtype=torch.bfloat16, device=q.device) for _ in range(2))
+        dvalue = torch.empty_like(dout)
+        dg, dbeta = torch.empty(g_shape, dtype=torch.float32, device=q.device), torch.empty_like(beta)
+        _lib.check(_lib.get_lib().flb_delta_bwd(
+            q.data_ptr(), k.data_ptr(), q.stride(0), k.stride(0), beta.data_ptr(), heads, repeat, dk, dv, int(channel), int(normalize), scale,
+            chunk.data_ptr(), doc_chunk.data_ptr(), docs, chunks, decay.data_ptr(), norm_q.data_ptr(), norm_k.data_ptr(), tri_t.data_ptr(),
+            tri_p.data_ptr(), tri_n.data_ptr(), _lib.ptr(k_in), _lib.ptr(k_out), _lib.ptr(q_in), u.data_ptr(), state.data_ptr(), dout.data_ptr(),
+            dr.data_ptr(), dstate.data_ptr(), dq.data_ptr(), dkey.data_ptr(), dvalue.data_ptr(), dg.data_ptr(), dbeta.data_ptr(), _lib.stream_ptr()),
+            "flb_delta_bwd")
+        _lib.count_launch(2)
+        if repeat > 1:
+            dq, dkey = (t.view(tokens, key_heads, repeat, dk).sum(2) for t in (dq, dkey))
+        return dq, dkey, dvalue, dg, dbeta, None, None, None
+
+
 def chunk_delta_rule(q, k, v, g, beta, cu_seqlens=None, chunk: int = 64, normalize_qk: bool = True, scale: float | None = None) -> torch.Tensor:
-    """q, k [tokens, heads, dk]; v [tokens, heads, dv]; g [tokens, heads(, dk)] log decay; beta [tokens, heads] -> [tokens, heads, dv]."""
+    """q, k [tokens, heads, dk] (or fewer heads, each serving as many adjacent heads of v); v [tokens, heads, dv]; g [tokens, heads(, dk)]
+    log decay; beta [tokens, heads] -> [tokens, heads, dv].  bf16 CUDA inputs with heads of 64 or 128 run `csrc/delta.cu`."""
+    if _DeltaRule.applies(q, k, v, g, beta):
+        return _DeltaRule.apply(q, k, v, g, beta, cu_seqlens, normalize_qk, float(q.shape[-1] ** -0.5 if scale is None else scale))
+    if (repeat := v.shape[1] // q.shape[1]) > 1:
+        q, k = q.repeat_interleave(repeat, dim=1), k.repeat_interleave(repeat, dim=1)
     if normalize_qk:
         q, k = l2_normalize(q.float()), l2_normalize(k.float())
     q = q * (q.shape[-1] ** -0.5 if scale is None else scale)

@@ -798,3 +798,55 @@ def test_delta_rule_state_scan_kernel(per_channel):
     assert _rel_err(out, reference) < 1e-2
     for name, a, b in zip("q k v g beta".split(), grads, reference_grads):
         assert _rel_err(a, b) < 1e-2, name
+
+
+@pytest.mark.parametrize("per_channel", [False, True])
+@pytest.mark.parametrize("tokens, boundaries, heads, key_heads, dk, dv, normalize", [
+    (1, None, 2, 2, 64, 64, True),  # one token
+    (65, None, 2, 1, 128, 128, True),  # one token behind a whole chunk, two value heads per key head
+    (200, [0, 64, 64, 127, 191], 4, 2, 64, 128, True),  # an empty document, chunk edges, padding behind the last document
+    (320, [0, 1, 300, 320], 3, 3, 128, 64, False),
+])
+def test_delta_rule_kernels(per_channel, tokens, boundaries, heads, key_heads, dk, dv, normalize):
+    """`csrc/delta.cu` against the token-by-token fp32 restatement: q, k, v as strided slices of one projection."""
+    from fast_llm_b200.ops.ssm import _DeltaRule, chunk_delta_rule, delta_rule_reference
+
+    torch.manual_seed(0)
+    dev = "cuda"
+    packed = torch.randn(tokens, 2 * key_heads * dk + heads * dv, device=dev).bfloat16().requires_grad_()
+    g = (-torch.rand((tokens, heads, dk) if per_channel else (tokens, heads), device=dev) * 2).requires_grad_()  # decays down to exp(-2) per token
+    beta = torch.rand(tokens, heads, device=dev).requires_grad_()
+    cu = None if boundaries is None else torch.tensor(boundaries, device=dev, dtype=torch.int32)
+    grad_out = torch.randn(tokens, heads, dv, device=dev).bfloat16()
+    scale = 1.0 if normalize else 0.1  # raw keys: keep the recurrence contracting
+    rows = [key_heads * dk, key_heads * dk, heads * dv]
+
+    def split(t):
+        q, k, v = t.split(rows, dim=-1)
+        return (q * 1).unflatten(-1, (key_heads, dk)), k.unflatten(-1, (key_heads, dk)), v.unflatten(-1, (heads, dv))
+
+    def run(fn, p, g, b):
+        q, k, v = split(p)
+        return fn(q, k if normalize else k * 0.05, v, g, b)
+
+    q, k, v = split(packed)
+    assert _DeltaRule.applies(q, k, v, g, beta)
+    out = run(lambda *t: chunk_delta_rule(*t, cu, normalize_qk=normalize, scale=scale), packed, g, beta)
+    grads = torch.autograd.grad(out, (packed, g, beta), grad_out)
+    inputs = [t.detach().float().requires_grad_() for t in (packed, g, beta)]
+
+    def reference(q, k, v, g, b):
+        if not normalize:
+            k = k.detach().bfloat16().float() + (k - k.detach())  # the value the kernel gets
+        repeat = heads // key_heads
+        return delta_rule_reference(q.repeat_interleave(repeat, 1), k.repeat_interleave(repeat, 1), v, g, b, cu, normalize_qk=normalize, scale=scale)
+
+    ref = run(reference, *inputs)
+    ref_grads = torch.autograd.grad(ref, inputs, grad_out.float())
+    # bf16 results carry one rounding (2^-9 of a value, two where value heads share a key head); the rest is fp32 throughout
+    assert _rel_err(out, ref) < 3e-3
+    assert _rel_err(grads[0], ref_grads[0]) < 6e-3
+    # The decay gradient is a difference of row products of up to dk terms each, 2^-24 relative: where the exact value is zero (the first
+    # token of a document) dk * 2^-24 < 1e-5 of products of order one stays behind.
+    for name, a, b in zip(["g", "beta"], grads[1:], ref_grads[1:]):
+        assert float((a - b).norm()) < 1e-3 * float(b.norm()) + 1e-5 * b.numel() ** 0.5, name

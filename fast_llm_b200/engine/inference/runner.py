@@ -12,17 +12,63 @@ class KeyValueCache:
     """Generation cache of an attention-only decoder.  Per attention layer, in layer order: the rotated keys and values of
     every row's positions so far, `[rows * length, width]` with the rows one after another (a row's left padding included:
     it is a document of its own, as in the packed forward pass).  Parity: the `past_key_values` / `presents` lists of
-    `fast_llm/models/gpt/huggingface.py:158-199`."""
+    `fast_llm/models/gpt/huggingface.py:158-199`.
+
+    Generation steps append to one buffer `[layers, rows, capacity, width]` that grows by doubling, so a step writes its own
+    position instead of copying all earlier ones."""
 
     def __init__(self, pads: list[int]):
         self.pads = list(pads)  # left padding of every row
-        self.layers: list[torch.Tensor] = []
         self.length = 0  # positions held per row
         self.on_reorder = None  # called with the row index before a reorder (tensor-parallel workers follow it)
+        self._layers: list[torch.Tensor] = []
+        self._buffer: torch.Tensor | None = None  # holds the positions instead of `_layers` once a step has reserved it
+        self._device_pads: torch.Tensor | None = None
 
     @property
     def rows(self) -> int:
         return len(self.pads)
+
+    @property
+    def width(self) -> int | None:
+        """Elements per position of a layer, None while empty or if the layers differ."""
+        if self._buffer is not None:
+            return self._buffer.shape[-1]
+        widths = {t.shape[-1] for t in self._layers}
+        return widths.pop() if len(widths) == 1 else None if not widths else -1
+
+    @property
+    def layers(self) -> list[torch.Tensor]:
+        if self._buffer is not None:
+            return [t[:, : self.length].reshape(self.rows * self.length, -1) for t in self._buffer.unbind(0)]
+        return self._layers
+
+    @layers.setter
+    def layers(self, layers: list[torch.Tensor]) -> None:
+        self._layers, self._buffer = list(layers), None
+
+    def reserve(self, length: int, layers: int, width: int, device) -> tuple[torch.Tensor, torch.Tensor]:
+        """(buffer with room for `length` positions of every row, left padding of the rows on the device)."""
+        if self._buffer is None or self._buffer.shape[2] < length:
+            buffer = torch.empty(layers, self.rows, -(-2 * length // 64) * 64, width, dtype=torch.bfloat16, device=device)
+            if self._buffer is not None:
+                buffer[:, :, : self.length] = self._buffer[:, :, : self.length]
+            else:
+                for i, kv in enumerate(self._layers):
+                    buffer[i, :, : self.length] = kv.view(self.rows, self.length, width)
+            self._buffer, self._layers = buffer, []
+        if self._device_pads is None:
+            self._device_pads = torch.tensor(self.pads, dtype=torch.int32, device=device)
+        return self._buffer, self._device_pads
+
+    def __copy__(self) -> "KeyValueCache":
+        """A branch of the generation: later steps of either cache do not show in the other."""
+        other = KeyValueCache(self.pads)
+        other.__dict__.update(self.__dict__)
+        other.pads, other._layers = list(self.pads), list(self._layers)
+        if self._buffer is not None:
+            other._buffer = self._buffer.clone()
+        return other
 
     def get_seq_length(self, layer_idx: int = 0) -> int:
         return self.length
@@ -36,9 +82,13 @@ class KeyValueCache:
     def reorder(self, index: torch.Tensor) -> None:
         """Beam search: row i continues from row index[i]."""
         order = index.tolist()
-        self.layers = [kv.view(self.rows, self.length, -1).index_select(0, index.to(kv.device)).reshape(len(order) * self.length, -1)
-                       for kv in self.layers]
+        if self._buffer is not None:
+            self._buffer = self._buffer.index_select(1, index.to(self._buffer.device))
+        else:
+            self._layers = [kv.view(self.rows, self.length, -1).index_select(0, index.to(kv.device)).reshape(len(order) * self.length, -1)
+                            for kv in self._layers]
         self.pads = [self.pads[i] for i in order]
+        self._device_pads = None
 
 
 class InferenceRunner:
@@ -104,6 +154,14 @@ class InferenceRunner:
         blocks = [layer.unwrap() for layer in self._model.base_model.get_layers() if isinstance(layer.unwrap(), DecoderBlock)]
         return bool(blocks) and all(type(block.mixer) is Attention and block.mixer._sdp_dim.size == 1 for block in blocks)
 
+    def _decode_plan(self):
+        """Description of the decoder for the native generation step, None if some part of it has to run layer by layer."""
+        if not hasattr(self, "_plan"):
+            from fast_llm_b200.engine.inference.decode import DecodePlan
+
+            self._plan = DecodePlan.build(self._model)
+        return self._plan
+
     @torch.no_grad()
     def forward_rows(self, tokens: torch.Tensor, cache: KeyValueCache, output_hidden_states=None):
         """`tokens` [rows, n]: the next n positions of every row of `cache` (the whole left-padded prompt when the cache is
@@ -112,6 +170,8 @@ class InferenceRunner:
 
         rows, new = tokens.shape
         assert rows == cache.rows
+        if not output_hidden_states and (plan := self._decode_plan()) is not None and plan.takes(rows, new, cache):
+            return plan.step(tokens, cache, self._distributed.device), {}
         held = cache.length
         cu_q, cu_k, positions, documents = [0], [0], [], []
         for pad in cache.pads:
@@ -140,7 +200,7 @@ class InferenceRunner:
             LanguageModelKwargs.sequence_k_offset: rows * (held + new), "max_position": held + new,
             LanguageModelKwargs.key_value_rows: rows, LanguageModelKwargs.presents: [], "return_logits": True,
         }
-        if cache.layers:
+        if held:
             kwargs[LanguageModelKwargs.past_key_values] = list(cache.layers)
         if output_hidden_states:
             kwargs["output_hidden_states"] = set(output_hidden_states)

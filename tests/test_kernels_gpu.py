@@ -850,3 +850,63 @@ def test_delta_rule_kernels(per_channel, tokens, boundaries, heads, key_heads, d
     # token of a document) dk * 2^-24 < 1e-5 of products of order one stays behind.
     for name, a, b in zip(["g", "beta"], grads[1:], ref_grads[1:]):
         assert float((a - b).norm()) < 1e-3 * float(b.norm()) + 1e-5 * b.numel() ** 0.5, name
+
+
+def _decoder(heads, kv_heads, head_size, hidden, ffn, vocab, norm, gated, window, bias):
+    import fast_llm_b200.models.auto  # noqa: F401
+    from fast_llm_b200.engine.inference.huggingface import HuggingfaceGPTModelForCausalLM
+    from fast_llm_b200.engine.multi_stage.config import StageMode
+    from fast_llm_b200.models.gpt.config import GPTModelConfig
+    from fast_llm_b200.models.gpt.model import GPTModel
+    from fast_llm_b200.parallel.distributed import Distributed
+
+    mixer = {"type": "attention", "rotary": {"type": "default"}, "heads": heads, "head_groups": kv_heads, "head_size": head_size, "add_linear_biases": bias}
+    if window:
+        mixer["window_size"] = window
+    config = GPTModelConfig.from_dict({
+        "base_model": {"embeddings": {"vocab_size": vocab}, "hidden_size": hidden,
+                       "decoder": {"num_blocks": 2, "block": {"mixer": mixer, "normalization": {"type": norm},
+                                                              "mlp": {"intermediate_size": ffn, "gated": gated, "add_linear_biases": bias}}},
+                       "head": {"normalization": {"type": norm}}},
+        "distributed": {"compute_dtype": "bf16", "world_size": 1, "rank": 0, "local_world_size": 1}})
+    config.validate()
+    model = GPTModel(config)
+    model.setup(Distributed(config.distributed), mode=StageMode.inference)
+    model.initialize_weights()
+    if bias:  # biases start at zero
+        for name in model.parameter_names:
+            if name.endswith("bias"):
+                model.import_state_tensor(name, "weights", torch.randn_like(next(t for n, _, t in model.get_state_tensor_iterator(("weights",)) if n == name)) * 0.1)
+        model.invalidate_buffers()
+    return HuggingfaceGPTModelForCausalLM(model)
+
+
+@pytest.mark.parametrize("rows, prompt, steps, shape", [
+    (1, 3, 4, dict(heads=4, kv_heads=2, head_size=64, hidden=256, ffn=512, vocab=512, norm="rms_norm", gated=True, window=0, bias=False)),
+    (9, 70, 3, dict(heads=16, kv_heads=1, head_size=64, hidden=512, ffn=1040, vocab=515, norm="layer_norm", gated=False, window=0, bias=True)),
+    (16, 130, 3, dict(heads=4, kv_heads=4, head_size=128, hidden=512, ffn=1536, vocab=1000, norm="rms_norm", gated=True, window=33, bias=False)),
+    (2, 1100, 2, dict(heads=8, kv_heads=1, head_size=128, hidden=1024, ffn=2048, vocab=1024, norm="rms_norm", gated=True, window=0, bias=False)),
+])
+def test_native_generation_step(rows, prompt, steps, shape):
+    """`csrc/decode.cu` against the packed forward pass over the whole prefix: left padding, cache growth, windows, biases, both norms."""
+    model = _decoder(**shape)
+    torch.manual_seed(0)
+    ids = torch.randint(1, shape["vocab"], (rows, prompt + steps), device="cuda")
+    mask = torch.ones(rows, prompt + steps, dtype=torch.int64, device="cuda")
+    for row in range(1, rows):
+        mask[row, : (row * 7) % max(prompt // 2, 1)] = 0
+    plan = model._inference_runner._decode_plan()
+    assert plan is not None
+    with torch.no_grad():
+        full = model(input_ids=ids, attention_mask=mask, use_cache=False).logits
+        out = model(input_ids=ids[:, :prompt], attention_mask=mask[:, :prompt], use_cache=True)
+        for step in range(steps):
+            assert plan.takes(rows, 1, out.past_key_values)
+            out = model(input_ids=ids[:, prompt + step : prompt + step + 1], past_key_values=out.past_key_values, use_cache=True)
+            assert out.logits.shape == (rows, 1, shape["vocab"])
+            # two bf16 evaluations of two blocks: a dozen roundings of 2^-9 each
+            assert _rel_err(out.logits[:, 0], full[:, prompt + step]) < 2e-2, step
+        # a later call with several tokens continues from the buffer through the layers
+        cache = out.past_key_values
+        more = model(input_ids=ids[:, :2], past_key_values=cache, use_cache=True)
+        assert more.logits.shape[1] == 2 and cache.get_seq_length() == prompt + steps + 2

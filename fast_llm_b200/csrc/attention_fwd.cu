@@ -1,5 +1,5 @@
 // Flash-attention forward on tcgen05 tensor cores: packed variable-length documents, causal + sliding window, GQA,
-// head size 128, bf16 in / bf16 out, fp32 softmax statistics.
+// head sizes up to 128 (tiles 64 or 128 wide), bf16 in / bf16 out, fp32 softmax statistics.
 //
 // One CTA owns TWO 128-row query tiles (256 consecutive rows) of one head of one document and walks the key/value tiles
 // (128 rows) either of them may see; the two query tiles share every K / V tile and alternate on the tensor pipe, so
@@ -13,8 +13,8 @@
 //               2^8 (lazy rescaling); finally O / l is written out with the row's log-sum-exp.
 // All mbarrier waits are bounded (error word).
 //
-// Layout contract: `qkv` rows hold [q heads | k heads | v heads] x 128 (any row stride that is a multiple of 8
-// elements); out rows hold heads x 128; lse is [heads, total_tokens] fp32 (natural log), the layout the backward expects.
+// Layout contract: `qkv` rows hold [q heads | k heads | v heads] x head size (a multiple of 8; any row stride that is a multiple of
+// 8 elements); out rows hold heads x head size; lse is [heads, total_tokens] fp32 (natural log), the layout the backward expects.
 #include "tcgen05.cuh"
 #include <cstdlib>
 #include <mutex>
@@ -56,6 +56,7 @@ struct AttnParams {
   int heads, kv_heads, q_col0, k_col0, v_col0;  // column (element) offsets of the q / k / v blocks inside a row
   int blocks_per_doc;    // ceil(max_seqlen_q / (2 * BM))
   int causal, window;    // window <= 0: unlimited; else a query sees the `window` most recent keys including itself
+  int head_dim;          // elements of a head in memory, at most the tile's width
   float scale_log2;      // softmax scale * log2(e)
   int* err_word;
 };
@@ -336,9 +337,15 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
 //   * the freed shared memory double-buffers V.
 // Barriers: 0-1 q_full[t], 2-3 k_full[s], 4-5 k_empty[s], 6-7 v_full[s], 8-9 v_empty[s], 10-11 s_full[t],
 //           12-13 p_full[t] (four warps), 14-15 pv_done[t].
-constexpr int SMEM2_Q = 0, SMEM2_K = 2 * TILE_BYTES_ATTN, SMEM2_V = 4 * TILE_BYTES_ATTN;
-constexpr int SMEM2_BARS = 6 * TILE_BYTES_ATTN;
-constexpr int SMEM2_TOTAL = SMEM2_BARS + 256 + 1024;
+//
+// HD: width of the head tiles, 128 or 64 (half the operand bytes and MMA time).  The tensor maps see [row][head][head_dim]: a head
+// narrower than the tile is filled with zeros by the copy, which change neither the scores nor the head_dim columns that are
+// written, so no padded copy of q, k, v exists (those copies and their gradients' were a fifth of a step with heads of 64).
+template <int HD>
+struct Fwd2 {
+  static constexpr int TILE = 128 * HD * 2, PANELS = HD / 64;
+  static constexpr int Q = 0, K = 2 * TILE, V = 4 * TILE, BARS = 6 * TILE, TOTAL = BARS + 256 + 1024;
+};
 
 // 2^x for x <= 8 on the FMA pipe: x = n + f with n = round(x) taken from the mantissa of x + 1.5 * 2^23, 2^f by a cubic
 // (relative error below 1e-4, well under the bf16 rounding of the probabilities it feeds), 2^n by adding n to the exponent field.
@@ -361,16 +368,19 @@ __device__ __forceinline__ void umma_bf16_ts(uint32_t tmem_d, uint32_t tmem_a, u
       : "memory");
 }
 
+template <int HD>
 __global__ void __launch_bounds__(kThreadsAttn, 1)
-attn_fwd_kernel_v2(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_kv, const AttnParams p) {
+attn_fwd_kernel_v2(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k, const __grid_constant__ CUtensorMap tmap_v,
+                   const AttnParams p) {
+  using C = Fwd2<HD>;
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw_addr = smem_u32(smem_raw);
   const uint32_t pad = (1024u - (raw_addr & 1023u)) & 1023u;
   uint8_t* smem = smem_raw + pad;
   const uint32_t sbase = raw_addr + pad;
-  const uint32_t bar0 = sbase + SMEM2_BARS;
+  const uint32_t bar0 = sbase + C::BARS;
   auto bar = [&](int i) { return bar0 + 8u * i; };
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + SMEM2_BARS + 8 * 16);
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + C::BARS + 8 * 16);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -393,7 +403,8 @@ attn_fwd_kernel_v2(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
 
   if (threadIdx.x == 0) {
     asm volatile("prefetch.tensormap [%0];" ::"l"(&tmap_q) : "memory");
-    asm volatile("prefetch.tensormap [%0];" ::"l"(&tmap_kv) : "memory");
+    asm volatile("prefetch.tensormap [%0];" ::"l"(&tmap_k) : "memory");
+    asm volatile("prefetch.tensormap [%0];" ::"l"(&tmap_v) : "memory");
     for (int i = 0; i <= 11; ++i) mbar_init(bar(i), 1);
     mbar_init(bar(12), 4); mbar_init(bar(13), 4);
     mbar_init(bar(14), 1); mbar_init(bar(15), 1);
@@ -415,9 +426,9 @@ attn_fwd_kernel_v2(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
     if (lane == 0) {
       // ---- producer
       for (int t = 0; t < num_q; ++t) {
-        mbar_expect_tx(bar(t), TILE_BYTES_ATTN);
-        for (int c = 0; c < 2; ++c)
-          tma_load_2d(sbase + SMEM2_Q + t * TILE_BYTES_ATTN + c * PANEL_BYTES, &tmap_q, bar(t), p.q_col0 + head * D + c * 64, q_begin + q0 + t * BM);
+        mbar_expect_tx(bar(t), C::TILE);
+        for (int c = 0; c < C::PANELS; ++c)
+          tma_load_3d(sbase + C::Q + t * C::TILE + c * PANEL_BYTES, &tmap_q, bar(t), c * 64, head, q_begin + q0 + t * BM);
       }
       bool ok = true;
       for (int j = 0; j < num_tiles && ok; ++j) {
@@ -425,30 +436,30 @@ attn_fwd_kernel_v2(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
         const uint32_t ph = (j >> 1) & 1;
         const int row = k_begin + (tile_lo + j) * BN;
         if (!mbar_wait(bar(4 + s), ph ^ 1u, abort_flag, p.err_word, 21)) { ok = false; break; }
-        mbar_expect_tx(bar(2 + s), TILE_BYTES_ATTN);
-        for (int c = 0; c < 2; ++c)
-          tma_load_2d(sbase + SMEM2_K + s * TILE_BYTES_ATTN + c * PANEL_BYTES, &tmap_kv, bar(2 + s), p.k_col0 + kv_head * D + c * 64, row);
+        mbar_expect_tx(bar(2 + s), C::TILE);
+        for (int c = 0; c < C::PANELS; ++c)
+          tma_load_3d(sbase + C::K + s * C::TILE + c * PANEL_BYTES, &tmap_k, bar(2 + s), c * 64, kv_head, row);
         if (!mbar_wait(bar(8 + s), ph ^ 1u, abort_flag, p.err_word, 22)) { ok = false; break; }
-        mbar_expect_tx(bar(6 + s), TILE_BYTES_ATTN);
-        for (int c = 0; c < 2; ++c)
-          tma_load_2d(sbase + SMEM2_V + s * TILE_BYTES_ATTN + c * PANEL_BYTES, &tmap_kv, bar(6 + s), p.v_col0 + kv_head * D + c * 64, row);
+        mbar_expect_tx(bar(6 + s), C::TILE);
+        for (int c = 0; c < C::PANELS; ++c)
+          tma_load_3d(sbase + C::V + s * C::TILE + c * PANEL_BYTES, &tmap_v, bar(6 + s), c * 64, kv_head, row);
       }
     }
   } else if (warp == 1) {
     if (lane == 0) {
       // ---- MMA issuer
       constexpr uint32_t idesc_qk = make_idesc(BM, BN, false, false);
-      constexpr uint32_t idesc_pv = make_idesc(BM, D, false, true);
+      constexpr uint32_t idesc_pv = make_idesc(BM, HD, false, true);
       bool ok = true;
       auto issue_qk = [&](int t, int j) -> bool {
         const int s = j & 1;
         if (t == 0 && !mbar_wait(bar(2 + s), (j >> 1) & 1, abort_flag, p.err_word, 24)) return false;  // K_j landed
         tc_fence_after();
 #pragma unroll
-        for (int k = 0; k < D / UMMA_K; ++k) {
+        for (int k = 0; k < HD / UMMA_K; ++k) {
           const uint32_t off = (k >> 2) * PANEL_BYTES + (k & 3) * 32;
-          umma_bf16(tmem + t * 128, make_smem_desc(sbase + SMEM2_Q + t * TILE_BYTES_ATTN + off, 16, 1024),
-                    make_smem_desc(sbase + SMEM2_K + s * TILE_BYTES_ATTN + off, 16, 1024), idesc_qk, k != 0);
+          umma_bf16(tmem + t * 128, make_smem_desc(sbase + C::Q + t * C::TILE + off, 16, 1024),
+                    make_smem_desc(sbase + C::K + s * C::TILE + off, 16, 1024), idesc_qk, k != 0);
         }
         umma_commit(bar(10 + t));                      // S_t(j) ready (and every earlier MMA of this thread complete)
         if (t == num_q - 1) umma_commit(bar(4 + s));   // K slot free
@@ -467,7 +478,7 @@ attn_fwd_kernel_v2(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
 #pragma unroll
           for (int k = 0; k < BN / UMMA_K; ++k)
             umma_bf16_ts(tmem + 256 + t * 128, tmem + t * 128 + k * 8,
-                         make_smem_desc(sbase + SMEM2_V + s * TILE_BYTES_ATTN + k * 2048, PANEL_BYTES, 1024), idesc_pv, (j | k) != 0);
+                         make_smem_desc(sbase + C::V + s * C::TILE + k * 2048, PANEL_BYTES, 1024), idesc_pv, (j | k) != 0);
           umma_commit(bar(14 + t));                     // O_t updated
           if (t == num_q - 1) umma_commit(bar(8 + s));  // V slot free
           // S_t of the next key tile goes behind it: the pipe runs this thread's MMAs in order, so P_t(j) is consumed first
@@ -524,7 +535,7 @@ attn_fwd_kernel_v2(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
       // S_t(j) being complete means O_t += P_t(j - 1) V is complete too (same issuing thread, earlier in its order)
       if (j > 0 && __any_sync(0xffffffffu, alpha != 1.f)) {
 #pragma unroll 1
-        for (int c = 0; c < 4; ++c) {
+        for (int c = 0; c < HD / 32; ++c) {
           uint32_t o[32];
           tmem_ld32(tmem_o + c * 32, o);
           tmem_wait_ld();
@@ -571,9 +582,9 @@ attn_fwd_kernel_v2(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
       tc_fence_after();
       const bool valid_row = qi < q_len;
       const float inv_l = (l > 0.f) ? 1.f / l : 0.f;
-      __nv_bfloat16* orow = p.out + ((long long)(q_begin + qi) * p.heads + head) * D;
+      __nv_bfloat16* orow = p.out + ((long long)(q_begin + qi) * p.heads + head) * p.head_dim;
 #pragma unroll 1
-      for (int c = 0; c < 4; ++c) {
+      for (int c = 0; c < HD / 32; ++c) {
         uint32_t o[32];
         if (num_tiles > 0 && ok) {
           tmem_ld32(tmem_o + c * 32, o);
@@ -585,6 +596,7 @@ attn_fwd_kernel_v2(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
         if (valid_row) {
 #pragma unroll
           for (int g = 0; g < 4; ++g) {
+            if (c * 32 + g * 8 >= p.head_dim) break;
             float f[8];
 #pragma unroll
             for (int i = 0; i < 8; ++i) f[i] = __uint_as_float(o[g * 8 + i]) * inv_l;
@@ -631,6 +643,23 @@ bool row_tmap(CUtensorMap* map, const void* base, uint64_t cols, uint64_t rows, 
   }
   return res == CUDA_SUCCESS;
 }
+// Three-dimensional view [row][head][head_dim] of the heads that start at `base`; boxes of 128 rows x 64 columns of one head.
+bool head_tmap(CUtensorMap* map, const void* base, int head_dim, int heads, uint64_t rows, uint64_t row_stride_elems) {
+  EncodeTiledFn enc = encode_fn();
+  if (!enc) return false;
+  cuuint64_t dims[3] = {(cuuint64_t)head_dim, (cuuint64_t)heads, rows};
+  cuuint64_t strides[2] = {(cuuint64_t)head_dim * 2, row_stride_elems * 2};
+  cuuint32_t box[3] = {64, 1, 128};
+  cuuint32_t es[3] = {1, 1, 1};
+  CUresult res = CUDA_SUCCESS;
+  for (int attempt = 0; attempt < 2; ++attempt) {
+    res = enc(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(base), dims, strides, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE,
+              CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (res != CUDA_ERROR_INVALID_CONTEXT) break;
+    cudaFree(nullptr);  // a thread that made no runtime call yet has no current context: bind the primary one
+  }
+  return res == CUDA_SUCCESS;
+}
 // 0: P kept in tensor memory (default); 1: the first kernel, P through shared memory.  FLB_ATTENTION_FWD=smem presets 1.
 int g_forward_variant = [] { const char* v = getenv("FLB_ATTENTION_FWD"); return (v && v[0] == 's') ? 1 : 0; }();
 
@@ -648,37 +677,49 @@ int* attn_err_word() {
 }
 }  // namespace
 
-// q rows: [total_q, q_stride] with query head h at columns q_col0 + h*128; kv rows: [total_k, kv_stride] with key head g at
-// k_col0 + g*128 and value head g at v_col0 + g*128 (q and kv may be the same packed tensor).  head size must be 128.
+// q rows: [total_q, q_stride] with query head h at columns q_col0 + h*head_dim; kv rows: [total_k, kv_stride] with key head g at
+// k_col0 + g*head_dim and value head g at v_col0 + g*head_dim (q and kv may be the same packed tensor).  head_dim: a multiple of 8,
+// at most 128; up to 64 the 64-wide tiles are used.
 FLB_API int flb_attention_fwd(const void* q, long long q_stride, int q_col0, const void* kv, long long kv_stride, int k_col0,
                               int v_col0, const int* cu_q, const int* cu_k, int batch, int max_seqlen_q, long long total_q,
                               long long total_k, int heads, int kv_heads, int head_dim, void* out, float* lse, int causal, int window,
                               float softmax_scale, cudaStream_t stream) {
-  if (head_dim != D || heads % kv_heads || q_stride % 8 || kv_stride % 8 || batch <= 0) return FLB_ERR_SHAPE;
+  if (head_dim <= 0 || head_dim > D || head_dim % 8 || heads % kv_heads || q_stride % 8 || kv_stride % 8 || batch <= 0) return FLB_ERR_SHAPE;
   if ((reinterpret_cast<uintptr_t>(q) & 15) || (reinterpret_cast<uintptr_t>(kv) & 15) || (q_col0 % 8) || (k_col0 % 8) || (v_col0 % 8))
     return FLB_ERR_SHAPE;
-  CUtensorMap tq, tkv;
-  if (!row_tmap(&tq, q, (uint64_t)q_stride, (uint64_t)total_q, (uint64_t)q_stride)) return FLB_ERR_TMA;
-  if (!row_tmap(&tkv, kv, (uint64_t)kv_stride, (uint64_t)total_k, (uint64_t)kv_stride)) return FLB_ERR_TMA;
+  const bool p_in_smem = g_forward_variant == 1 && head_dim == D;
+  CUtensorMap tq, tk, tv;
+  const __nv_bfloat16 *qp = (const __nv_bfloat16*)q, *kvp = (const __nv_bfloat16*)kv;
+  if (p_in_smem) {
+    if (!row_tmap(&tq, q, (uint64_t)q_stride, (uint64_t)total_q, (uint64_t)q_stride)) return FLB_ERR_TMA;
+    if (!row_tmap(&tk, kv, (uint64_t)kv_stride, (uint64_t)total_k, (uint64_t)kv_stride)) return FLB_ERR_TMA;
+  } else {
+    if (!head_tmap(&tq, qp + q_col0, head_dim, heads, (uint64_t)total_q, (uint64_t)q_stride)) return FLB_ERR_TMA;
+    if (!head_tmap(&tk, kvp + k_col0, head_dim, kv_heads, (uint64_t)total_k, (uint64_t)kv_stride)) return FLB_ERR_TMA;
+    if (!head_tmap(&tv, kvp + v_col0, head_dim, kv_heads, (uint64_t)total_k, (uint64_t)kv_stride)) return FLB_ERR_TMA;
+  }
   static bool configured = false;
   if (!configured) {
     cudaError_t e = cudaFuncSetAttribute(attn_fwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_TOTAL);
     if (e != cudaSuccess) return flb_record_cuda_error(e);
-    e = cudaFuncSetAttribute(attn_fwd_kernel_v2, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM2_TOTAL);
+    e = cudaFuncSetAttribute(attn_fwd_kernel_v2<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, Fwd2<128>::TOTAL);
+    if (e != cudaSuccess) return flb_record_cuda_error(e);
+    e = cudaFuncSetAttribute(attn_fwd_kernel_v2<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, Fwd2<64>::TOTAL);
     if (e != cudaSuccess) return flb_record_cuda_error(e);
     configured = true;
   }
-  const bool p_in_smem = g_forward_variant == 1;
   AttnParams p;
   p.cu_q = cu_q; p.cu_k = cu_k; p.out = (__nv_bfloat16*)out; p.lse = lse; p.total_q = total_q;
   p.heads = heads; p.kv_heads = kv_heads; p.q_col0 = q_col0; p.k_col0 = k_col0; p.v_col0 = v_col0;
   p.blocks_per_doc = (max_seqlen_q + 2 * BM - 1) / (2 * BM);
+  p.head_dim = head_dim;
   p.causal = causal; p.window = window; p.scale_log2 = softmax_scale * 1.4426950408889634f;
   p.err_word = attn_err_word();
   if (!p.err_word) return FLB_ERR_CUDA;
   dim3 grid(p.blocks_per_doc * batch, heads);
-  if (p_in_smem) attn_fwd_kernel<<<grid, kThreadsAttn, SMEM_TOTAL, stream>>>(tq, tkv, p);
-  else attn_fwd_kernel_v2<<<grid, kThreadsAttn, SMEM2_TOTAL, stream>>>(tq, tkv, p);
+  if (p_in_smem) attn_fwd_kernel<<<grid, kThreadsAttn, SMEM_TOTAL, stream>>>(tq, tk, p);
+  else if (head_dim > 64) attn_fwd_kernel_v2<128><<<grid, kThreadsAttn, Fwd2<128>::TOTAL, stream>>>(tq, tk, tv, p);
+  else attn_fwd_kernel_v2<64><<<grid, kThreadsAttn, Fwd2<64>::TOTAL, stream>>>(tq, tk, tv, p);
   FLB_CHECK_LAUNCH();
   return FLB_OK;
 }

@@ -5,8 +5,8 @@
 backward is a single GEMM.  `attention(q, k, v, ...)` is the general form (keys may include a prefix from earlier
 micro-sequences or other sequence-data-parallel ranks; causal masks are bottom-right aligned).
 
-On B200 both forms run this package's tcgen05 kernels (`csrc/attention_fwd.cu`, `csrc/attention_bwd.cu`: bf16, head size
-128, key segments at least as long as the query segments); smaller head sizes are zero-padded to 128.  Dropout, heads
+On B200 both forms run this package's tcgen05 kernels (`csrc/attention_fwd.cu`, `csrc/attention_bwd.cu`: bf16, head sizes up to
+128 that are a multiple of 8, key segments at least as long as the query segments).  Dropout, heads
 wider than 128, fp16 and a window without causality go through PyTorch's `scaled_dot_product_attention` per document.  On
 CPU a per-document PyTorch restatement, which doubles as the test oracle (math of `fast_llm/layers/attention/
 attention.py:209-256`).
@@ -72,7 +72,7 @@ def attention_backward_native(q2d, q_col0, kv2d, k_col0, v_col0, out, dout, lse,
     forward inputs have in `q2d` / `kv2d` (the gradient buffers mirror the input layout)."""
     total_q, total_k = q2d.shape[0], kv2d.shape[0]
     delta = torch.empty(heads, total_q, dtype=torch.float32, device=q2d.device)
-    dq_accum = torch.empty(heads * ((total_q + 31) // 32) * 32 * head_dim, dtype=torch.float32, device=q2d.device)
+    dq_accum = torch.empty(heads * ((total_q + 31) // 32) * 32 * (64 if head_dim <= 64 else 128), dtype=torch.float32, device=q2d.device)
     dout = dout.contiguous()
     _lib.check(
         _lib.get_lib().flb_attention_bwd(
@@ -83,12 +83,11 @@ def attention_backward_native(q2d, q_col0, kv2d, k_col0, v_col0, out, dout, lse,
     _lib.count_launch(3)
 
 
-_NATIVE_HEAD = 128  # head size of the tcgen05 kernels; smaller heads are zero-padded to it
-_MIN_ROWS = 128  # fewer query or key rows than one tile are padded with rows of no document
+_NATIVE_HEAD = 128  # widest head of the tcgen05 kernels
 
 
 def _joint_key_value_rows(k: torch.Tensor, v: torch.Tensor) -> torch.Tensor:
-    """[Tk, 2 * kv_heads * 128] rows holding the keys of every head followed by the values: a view when k and v already sit
+    """[Tk, 2 * kv_heads * head_dim] rows holding the keys of every head followed by the values: a view when k and v already sit
     side by side in one buffer (slices of a fused projection or of a gathered key/value tensor), else a copy."""
     tk, kv_heads, d = k.shape
     width = kv_heads * d
@@ -101,7 +100,7 @@ def _joint_key_value_rows(k: torch.Tensor, v: torch.Tensor) -> torch.Tensor:
 
 
 class _NativeAttention(KernelFunction):
-    """q [Tq, heads, 128], k / v [Tk, kv_heads, 128]; the key segments may be longer than the query segments (a prefix from
+    """q [Tq, heads, d], k / v [Tk, kv_heads, d]; the key segments may be longer than the query segments (a prefix from
     earlier micro-sequences or other sequence-data ranks): masks are bottom-right aligned."""
 
     @staticmethod
@@ -121,7 +120,7 @@ class _NativeAttention(KernelFunction):
     def backward(ctx, dout):
         q2d, kv2d, out, lse, cu_q, cu_k = ctx.saved_tensors
         max_k, heads, kv_heads, causal, window_size, scale = ctx.args
-        d = _NATIVE_HEAD
+        d = q2d.shape[1] // heads
         tq, tk, width = q2d.shape[0], kv2d.shape[0], kv_heads * d
         dq = torch.empty(tq, heads * d, dtype=q2d.dtype, device=q2d.device)
         # key rows outside every `cu_k` segment (another sequence-data rank's later tokens) are attended by no query here
@@ -133,12 +132,12 @@ class _NativeAttention(KernelFunction):
 
 
 class _PackedNativeAttention(KernelFunction):
-    """Self-attention over the fused projection output [tokens, (heads + 2 kv_heads) x 128]; the backward writes dq, dk and
+    """Self-attention over the fused projection output [tokens, (heads + 2 kv_heads) x d]; the backward writes dq, dk and
     dv into one packed gradient, so the projection's backward is one GEMM."""
 
     @staticmethod
     def forward(ctx, qkv, cu, max_len, heads, kv_heads, causal, window_size, scale):
-        d = _NATIVE_HEAD
+        d = qkv.shape[1] // (heads + 2 * kv_heads)
         nq, nkv = heads * d, kv_heads * d
         out, lse = attention_forward_native(qkv, 0, qkv, nq, nq + nkv, cu, cu, max_len, heads, kv_heads, d, causal, window_size, scale)
         ctx.save_for_backward(qkv, out, lse, cu)
@@ -149,7 +148,7 @@ class _PackedNativeAttention(KernelFunction):
     def backward(ctx, dout):
         qkv, out, lse, cu = ctx.saved_tensors
         max_len, heads, kv_heads, causal, window_size, scale = ctx.args
-        d = _NATIVE_HEAD
+        d = qkv.shape[1] // (heads + 2 * kv_heads)
         nq, nkv = heads * d, kv_heads * d
         dqkv = torch.empty_like(qkv)
         attention_backward_native(qkv, 0, qkv, nq, nq + nkv, out, dout.reshape(qkv.shape[0], nq), lse, cu, cu, max_len, heads, kv_heads, d,
@@ -195,16 +194,7 @@ def attention(q, k, v, cu_seqlens_q, cu_seqlens_k, max_seqlen_q: int, max_seqlen
         return attention_reference(q, k, v, cu_seqlens_q, cu_seqlens_k, causal, window_size, scale)
     if not (_native_dtype_ok(q, dropout_p) and d <= _NATIVE_HEAD and d % 8 == 0 and _kernel_supports(causal, window_size)):
         return _sdpa_fallback(q, k, v, cu_seqlens_q, cu_seqlens_k, causal, window_size, scale, dropout_p)
-    tq = q.shape[0]
-    # generation steps hold a few rows only: the tensor maps always cover at least one full 128-row tile (rows past the last
-    # `cu_seqlens` entry belong to no document: nothing reads or writes them)
-    rows_q, rows_k = max(_MIN_ROWS - tq, 0), max(_MIN_ROWS - k.shape[0], 0)
-    if d < _NATIVE_HEAD or rows_q or rows_k:
-        # zero columns change neither the scores nor the first d output columns
-        q = torch.nn.functional.pad(q, (0, _NATIVE_HEAD - d, 0, 0, 0, rows_q))
-        k, v = (torch.nn.functional.pad(t, (0, _NATIVE_HEAD - d, 0, 0, 0, rows_k)) for t in (k, v))
-    out = _NativeAttention.apply(q, k, v, cu_seqlens_q.int(), cu_seqlens_k.int(), max_seqlen_q, max_seqlen_k, causal, window_size, scale)
-    return out[:tq, :, :d] if (d < _NATIVE_HEAD or rows_q) else out
+    return _NativeAttention.apply(q, k, v, cu_seqlens_q.int(), cu_seqlens_k.int(), max_seqlen_q, max_seqlen_k, causal, window_size, scale)
 
 
 def packed_attention(qkv, cu_seqlens, max_seqlen: int, heads: int, kv_heads: int, head_dim: int, *, causal: bool = True,
@@ -212,7 +202,7 @@ def packed_attention(qkv, cu_seqlens, max_seqlen: int, heads: int, kv_heads: int
     scale = head_dim**-0.5 if scale is None else scale
     t = qkv.shape[0]
     nq, nkv = heads * head_dim, kv_heads * head_dim
-    if qkv.is_cuda and _native_dtype_ok(qkv, dropout_p) and head_dim == _NATIVE_HEAD and _kernel_supports(causal, window_size) \
+    if qkv.is_cuda and _native_dtype_ok(qkv, dropout_p) and head_dim <= _NATIVE_HEAD and head_dim % 8 == 0 and _kernel_supports(causal, window_size) \
             and qkv.stride(-1) == 1 and qkv.stride(0) % 8 == 0 and qkv.data_ptr() % 16 == 0:
         return _PackedNativeAttention.apply(qkv, cu_seqlens.int(), max_seqlen, heads, kv_heads, causal, window_size, scale)
     q = qkv[:, :nq].reshape(t, heads, head_dim)

@@ -910,3 +910,30 @@ def test_native_generation_step(rows, prompt, steps, shape):
         cache = out.past_key_values
         more = model(input_ids=ids[:, :2], past_key_values=cache, use_cache=True)
         assert more.logits.shape[1] == 2 and cache.get_seq_length() == prompt + steps + 2
+
+
+@pytest.mark.parametrize("doc_lengths, heads, kv_heads, d, window", [
+    ([5], 2, 1, 32, None),  # fewer rows than one tile, a head narrower than the 64-wide tile
+    ([130, 1, 257], 4, 4, 64, None),
+    ([300, 84], 4, 2, 64, 100),
+    ([129], 3, 1, 8, None),
+    ([200, 56], 2, 2, 96, None),  # narrower than the 128-wide tile
+])
+def test_packed_attention_head_sizes(doc_lengths, heads, kv_heads, d, window):
+    """Heads narrower than the tiles: the copy fills them with zeros and only the head's columns are written, forward and backward."""
+    from fast_llm_b200.ops.attention import attention_reference, packed_attention
+
+    torch.manual_seed(4)
+    total, nq, nkv = sum(doc_lengths), heads * d, kv_heads * d
+    qkv = torch.randn(total, nq + 2 * nkv, device="cuda", dtype=torch.bfloat16, requires_grad=True)
+    cu = torch.tensor([0] + list(torch.tensor(doc_lengths).cumsum(0)), device="cuda", dtype=torch.int32)
+    out = packed_attention(qkv, cu, max(doc_lengths), heads, kv_heads, d, causal=True, window_size=window)
+    g = torch.randn_like(out)
+    out.backward(g)
+    x = qkv.detach().float().requires_grad_()
+    ref = attention_reference(x[:, :nq].reshape(total, heads, d), x[:, nq : nq + nkv].reshape(total, kv_heads, d), x[:, nq + nkv :].reshape(total, kv_heads, d),
+                              cu, cu, True, window, d**-0.5).reshape(total, nq)
+    ref.backward(g.float())
+    # P and dS enter the second product rounded to bf16, as in the 128-wide cases above
+    assert _rel_err(out, ref) < 1.5e-2
+    assert torch.isfinite(qkv.grad).all() and _rel_err(qkv.grad, x.grad) < 2e-2

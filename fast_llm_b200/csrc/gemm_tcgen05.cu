@@ -221,14 +221,20 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
 // CTA-pair kernel: clusters of two CTAs, 256 x 256 tiles, tcgen05.mma.cta_group::2 issued by the leader (cluster rank 0)
 // ------------------------------------------------------------------------------------------------
 constexpr int PairTileM = 256, PairTileN = 256;
+// The gated epilogue turns every accumulator pair into three outputs and an exponential: with four warps per CTA it took 20 us per
+// tile where the main loop of K = 2048 takes 9, so it gets eight (two per TMEM lane quarter, each half of the columns) and the
+// shared memory for their staging comes out of the operand ring (five stages instead of six).
+template <int EPI>
 struct PairCfg {
   static constexpr int TILE_M = PairTileM, TILE_N = PairTileN;
+  static constexpr int EPI_WARPS = EPI == EPI_GATED_BF16 ? 8 : 4;
+  static constexpr int THREADS = 64 + 32 * EPI_WARPS;
   static constexpr int A_BYTES = BLOCK_M * BLOCK_K * 2;        // this CTA's 128 rows of A
   static constexpr int B_BYTES = (TILE_N / 2) * BLOCK_K * 2;   // this CTA's half of the B tile
   static constexpr int STAGE_BYTES = A_BYTES + B_BYTES;        // 32 KiB
-  static constexpr int STAGES = 6;
+  static constexpr int STAGES = EPI_WARPS == 8 ? 5 : 6;
   static constexpr int RING_BYTES = STAGES * STAGE_BYTES;
-  static constexpr int TILE_BYTES = RING_BYTES + 4 * kEpiWarpBytes;  // operand ring + epilogue staging (4 warps)
+  static constexpr int TILE_BYTES = RING_BYTES + EPI_WARPS * kEpiWarpBytes;  // operand ring + epilogue staging
   static constexpr int BAR_BYTES = 256;
   static constexpr int SMEM_BYTES = TILE_BYTES + BAR_BYTES + 1024;
   static constexpr int TMEM_COLS = 2 * TILE_N;
@@ -309,64 +315,79 @@ __device__ __forceinline__ TileInfo grouped_tile(const GroupArgs& g, int tile, i
 }
 
 // Epilogue of the first GEMM of a gated MLP: the tile holds gate columns [n0, n0 + 128) in accumulator columns 0..127 and the
-// matching up columns in 128..255.  Per 64-column piece three stores leave the warp's staging buffers: the gate piece of h at
-// column n0 + c, the up piece of h at column half + n0 + c, and act(gate) * up at column n0 + c of the second matrix.  The
-// activation is evaluated on the bf16-rounded values, i.e. on what h holds, so a later recomputation from h reproduces it.
+// matching up columns in 128..255; this warp drains 64 of each, starting at column c.  Three stores leave its staging buffers: the
+// gate piece of h at column n0 + c, the up piece of h at column half + n0 + c (both only if h is kept), and act(gate) * up at column
+// n0 + c of the second matrix.  The activation is evaluated on the bf16-rounded values, i.e. on what h holds, so a later
+// recomputation from h reproduces it.  `drained` is called once the accumulators have been read.
+template <typename Act, typename Drained>
 __device__ __forceinline__ void epilogue_gated(const CUtensorMap* tmap_h, const CUtensorMap* tmap_act, uint8_t* warp_buf, uint32_t taddr, int row0,
-                                               int n0, int half, int M, int act_type, int lane, uint32_t& counter) {
-  auto rounded = [](uint32_t bits) { return __bfloat162float(__float2bfloat16_rn(__uint_as_float(bits))); };
-#pragma unroll 1
-  for (int c = 0; c < 128; c += 64) {
-    if (row0 >= M || n0 + c >= half) break;
-    // three staged pieces per 64 columns (gate, up, activation); the accumulator columns are re-read from tensor memory for
-    // each instead of being kept in registers (a 64-column read costs far less than the store it feeds)
+                                               int n0, int c, int half, int M, bool keep_h, int lane, Act&& act, Drained&& drained) {
+  if (row0 >= M || n0 + c >= half) {
+    drained();
+    return;
+  }
+  uint8_t* const gate_row = warp_buf + lane * 128;
+  uint8_t* const up_row = gate_row + 4096;
+  uint32_t packed[32];
+  if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");  // the previous tile's stores have left the buffers
+  __syncwarp();
 #pragma unroll
-    for (int which = 0; which < 3; ++which) {
-      uint8_t* buf = warp_buf + (counter & 1u) * 4096;
-      ++counter;
-      if (lane == 0) tma_store_wait_read_1();
-      __syncwarp();
-      uint8_t* row_ptr = buf + lane * 128;
+  for (int h = 0; h < 2; ++h) {
+    uint32_t g[32], u[32];
+    tmem_ld32(taddr + c + h * 32, g);
+    tmem_ld32(taddr + 128 + c + h * 32, u);
+    tmem_wait_ld();
+    if (h == 1) drained();
 #pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        uint32_t g[32], u[32];
-        if (which != 1) tmem_ld32(taddr + c + h * 32, g);
-        if (which != 0) tmem_ld32(taddr + 128 + c + h * 32, u);
-        tmem_wait_ld();
+    for (int j = 0; j < 4; ++j) {
+      uint32_t gp[4], up[4];
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          uint32_t pk[4];
-#pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            const int i = 8 * j + 2 * e;
-            float a, b;
-            if (which == 0) { a = rounded(g[i]); b = rounded(g[i + 1]); }
-            else if (which == 1) { a = rounded(u[i]); b = rounded(u[i + 1]); }
-            else { a = act_fwd(rounded(g[i]), act_type) * rounded(u[i]); b = act_fwd(rounded(g[i + 1]), act_type) * rounded(u[i + 1]); }
-            __nv_bfloat162 v = __floats2bfloat162_rn(a, b);
-            pk[e] = *reinterpret_cast<uint32_t*>(&v);
-          }
-          *reinterpret_cast<uint4*>(row_ptr + (((h * 4 + j) ^ (lane & 7)) << 4)) = make_uint4(pk[0], pk[1], pk[2], pk[3]);
-        }
+      for (int e = 0; e < 4; ++e) {
+        const int i = 8 * j + 2 * e;
+        __nv_bfloat162 gv = __floats2bfloat162_rn(__uint_as_float(g[i]), __uint_as_float(g[i + 1]));
+        __nv_bfloat162 uv = __floats2bfloat162_rn(__uint_as_float(u[i]), __uint_as_float(u[i + 1]));
+        gp[e] = *reinterpret_cast<uint32_t*>(&gv);
+        up[e] = *reinterpret_cast<uint32_t*>(&uv);
+        const float2 gf = __bfloat1622float2(gv), uf = __bfloat1622float2(uv);
+        __nv_bfloat162 av = __floats2bfloat162_rn(act(gf.x) * uf.x, act(gf.y) * uf.y);
+        packed[h * 16 + 4 * j + e] = *reinterpret_cast<uint32_t*>(&av);
       }
-      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-      __syncwarp();
-      if (lane == 0) {
-        if (which == 0) tma_store_2d(tmap_h, smem_u32(buf), n0 + c, row0);
-        else if (which == 1) tma_store_2d(tmap_h, smem_u32(buf), half + n0 + c, row0);
-        else tma_store_2d(tmap_act, smem_u32(buf), n0 + c, row0);
-        tma_store_commit();
+      if (keep_h) {
+        const int at = ((h * 4 + j) ^ (lane & 7)) << 4;
+        *reinterpret_cast<uint4*>(gate_row + at) = make_uint4(gp[0], gp[1], gp[2], gp[3]);
+        *reinterpret_cast<uint4*>(up_row + at) = make_uint4(up[0], up[1], up[2], up[3]);
       }
     }
+  }
+  if (keep_h) {
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    __syncwarp();
+    if (lane == 0) {
+      tma_store_2d(tmap_h, smem_u32(warp_buf), n0 + c, row0);
+      tma_store_commit();
+      tma_store_2d(tmap_h, smem_u32(warp_buf + 4096), half + n0 + c, row0);
+      tma_store_commit();
+      tma_store_wait_read_1();  // the gate piece has left the first buffer
+    }
+    __syncwarp();
+  }
+#pragma unroll
+  for (int j = 0; j < 8; ++j)
+    *reinterpret_cast<uint4*>(gate_row + ((j ^ (lane & 7)) << 4)) = make_uint4(packed[4 * j], packed[4 * j + 1], packed[4 * j + 2], packed[4 * j + 3]);
+  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+  __syncwarp();
+  if (lane == 0) {
+    tma_store_2d(tmap_act, smem_u32(warp_buf), n0 + c, row0);
+    tma_store_commit();
   }
 }
 
 template <bool A_MN, bool B_MN, int EPI, int GROUP>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kNumThreads, 1)
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PairCfg<EPI>::THREADS, 1)
 gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
                  const __grid_constant__ CUtensorMap tmap_c, int use_tma_c, void* __restrict__ Cv, int M, int N, int K, long long ldc,
                  int* __restrict__ err_word, const GroupArgs group, const __grid_constant__ CUtensorMap tmap_act, int act_type) {
-  using C = PairCfg;
+  using C = PairCfg<EPI>;
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw_addr = smem_u32(smem_raw);
   const uint32_t pad = (1024u - (raw_addr & 1023u)) & 1023u;
@@ -396,7 +417,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
     }
     for (int a = 0; a < 2; ++a) {
       mbar_init(tfull_bar(a), 1);
-      mbar_init(tempty_bar(a), 8);  // leader only: four epilogue warps of each CTA
+      mbar_init(tempty_bar(a), 2 * C::EPI_WARPS);  // leader only: the epilogue warps of both CTAs
     }
     *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -521,8 +542,9 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
       }
     }
   } else {
-    // ---------------- epilogue warps (2..5) of both CTAs: each drains its own 128 accumulator rows ----------------
+    // ---------------- epilogue warps of both CTAs: each CTA drains its own 128 accumulator rows ----------------
     const int q = warp & 3;
+    [[maybe_unused]] uint8_t* const warp_buf = smem + C::RING_BYTES + (warp - 2) * kEpiWarpBytes;
     int it = 0;
     bool ok = true;
     uint32_t epi_counter = 0;
@@ -534,25 +556,38 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
       tc_fence_after();
       const int row0 = ti.c_row0 + (int)cta_rank * BLOCK_M + q * 32;
       const uint32_t taddr = tmem_base + ((uint32_t)(q * 32) << 16) + acc * C::TILE_N;
+      auto drained = [&] {
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive_cluster(map_to_cta(tempty_bar(acc), 0));
+      };
+      if constexpr (kGated) {  // never empty: only whole row blocks of an expert are visited
+        const int c = ((warp - 2) >> 2) * 64;
+        const bool keep_h = Cv != nullptr;
+        if (act_type == 1)
+          epilogue_gated(&tmap_c, &tmap_act, warp_buf, taddr, row0, ti.n0 / 2, c, gated_half, M, keep_h, lane, [](float x) { return act_fwd(x, 1); }, drained);
+        else
+          epilogue_gated(&tmap_c, &tmap_act, warp_buf, taddr, row0, ti.n0 / 2, c, gated_half, M, keep_h, lane,
+                         [&](float x) { return act_fwd(x, act_type); }, drained);
+        continue;
+      }
       const bool empty = ti.num_kb == 0;  // grouped weight gradient of an expert without rows: the tile is zero
       if (empty) {
-        if constexpr (EPI == EPI_STORE_BF16 || EPI == EPI_STORE_F32 || EPI == EPI_GATED_BF16) {
+        if constexpr (EPI == EPI_STORE_BF16 || EPI == EPI_STORE_F32) {
           uint32_t zeros[32];
 #pragma unroll
           for (int i = 0; i < 32; ++i) zeros[i] = 0u;
 #pragma unroll 1
           for (int c = 0; c < C::TILE_N / 32; ++c) store_chunk<EPI>(zeros, Cv, row0 + lane, ti.n0 + c * 32, c_rows, N, ldc);
         }
-      } else if constexpr (kGated) {
-        epilogue_gated(&tmap_c, &tmap_act, smem + C::RING_BYTES + q * kEpiWarpBytes, taddr, row0, ti.n0 / 2, gated_half, M, act_type, lane, epi_counter);
       } else if (GROUP == kGroupScatter) {
         // the tile lies inside one chunk: its rows go to that rank's staging slot, addressed from the slot's first row
         const int chunk = ti.m0 / group.scatter_chunk_rows;
         const int first = chunk * group.scatter_chunk_rows;
-        epilogue_tma<EPI>(group.scatter_maps + chunk, smem + C::RING_BYTES + q * kEpiWarpBytes, taddr, C::TILE_N, row0 - first, ti.n0,
+        epilogue_tma<EPI>(group.scatter_maps + chunk, warp_buf, taddr, C::TILE_N, row0 - first, ti.n0,
                           min(group.scatter_chunk_rows, M - first), N, lane, epi_counter);
       } else if (use_tma_c) {
-        epilogue_tma<EPI>(&tmap_c, smem + C::RING_BYTES + q * kEpiWarpBytes, taddr, C::TILE_N, row0, ti.n0, c_rows, N, lane, epi_counter);
+        epilogue_tma<EPI>(&tmap_c, warp_buf, taddr, C::TILE_N, row0, ti.n0, c_rows, N, lane, epi_counter);
       } else {
 #pragma unroll 1
         for (int c = 0; c < C::TILE_N / 32; ++c) {
@@ -562,9 +597,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
           store_chunk<EPI>(r, Cv, row0 + lane, ti.n0 + c * 32, c_rows, N, ldc);
         }
       }
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive_cluster(map_to_cta(tempty_bar(acc), 0));
+      drained();
     }
     if (lane == 0) tma_store_wait_all();
   }
@@ -731,17 +764,17 @@ int launch_pair(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap&
   auto kern = gemm_pair_kernel<A_MN, B_MN, EPI, GROUP>;
   static bool configured = false;
   if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, PairCfg::SMEM_BYTES);
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, PairCfg<EPI>::SMEM_BYTES);
     if (e != cudaSuccess) return flb_record_cuda_error(e);
     configured = true;
   }
-  int tiles = ((M + PairCfg::TILE_M - 1) / PairCfg::TILE_M) * ((N + PairCfg::TILE_N - 1) / PairCfg::TILE_N);
-  if (EPI == EPI_GATED_BF16) tiles = ((M + PairCfg::TILE_M - 1) / PairCfg::TILE_M) * ((N / 2 + 127) / 128);
+  int tiles = ((M + PairTileM - 1) / PairTileM) * ((N + PairTileN - 1) / PairTileN);
+  if (EPI == EPI_GATED_BF16) tiles = ((M + PairTileM - 1) / PairTileM) * ((N / 2 + 127) / 128);
   if (GROUP == kGroupRows || GROUP == kGroupWgrad) tiles = tiles_upper_bound;
   int clusters = st->num_sms / 2;
   if (max_ctas > 1 && max_ctas / 2 < clusters) clusters = max_ctas / 2;
   if (tiles < clusters) clusters = tiles;
-  kern<<<2 * clusters, kNumThreads, PairCfg::SMEM_BYTES, stream>>>(ta, tb, tc, use_tc, C, M, N, K, ldc, st->err_word, group, tact ? *tact : tc, act_type);
+  kern<<<2 * clusters, PairCfg<EPI>::THREADS, PairCfg<EPI>::SMEM_BYTES, stream>>>(ta, tb, tc, use_tc, C, M, N, K, ldc, st->err_word, group, tact ? *tact : tc, act_type);
   FLB_CHECK_LAUNCH();
   return FLB_OK;
 }
@@ -893,7 +926,8 @@ FLB_API int flb_grouped_gemm_gated_bf16(const void* A, const void* W, void* H, v
 
 // First GEMM of a gated MLP fused with the activation: H[M, 2F] = A[M, K] W^T with W = [gate rows; up rows] stacked ([2F, K],
 // K contiguous), and ACT[M, F] = act(H[:, :F]) * H[:, F:], both bf16, from one pass over the accumulators (CTA-pair kernel).
-// F must be a multiple of 8 (TMA strides); rows and columns past M / F are clipped.  act_type: see activations.cuh.
+// F must be a multiple of 8 (TMA strides); rows and columns past M / F are clipped.  act_type: see activations.cuh.  H may be null
+// (no backward pass follows): two thirds of the output bytes stay unwritten.
 FLB_API int flb_gemm_gated_bf16(const void* A, const void* W, void* H, void* ACT, int M, int F, int K, long long lda, long long ldw,
                                 long long ldh, long long ldact, int act_type, cudaStream_t stream) {
   if (M <= 0 || F <= 0 || K <= 0) return FLB_ERR_SHAPE;
@@ -905,8 +939,9 @@ FLB_API int flb_gemm_gated_bf16(const void* A, const void* W, void* H, void* ACT
   CUtensorMap ta, tb, th, tact;
   if (!make_tmap(&ta, A, (uint64_t)K, (uint64_t)M, (uint64_t)lda, BLOCK_K, BLOCK_M)) return FLB_ERR_TMA;
   if (!make_tmap(&tb, W, (uint64_t)K, (uint64_t)2 * F, (uint64_t)ldw, BLOCK_K, 128u)) return FLB_ERR_TMA;
-  if (!make_tmap_c(&th, H, (uint64_t)2 * F, (uint64_t)M, (uint64_t)ldh, false)) return FLB_ERR_TMA;
   if (!make_tmap_c(&tact, ACT, (uint64_t)F, (uint64_t)M, (uint64_t)ldact, false)) return FLB_ERR_TMA;
+  if (H == nullptr) th = tact;  // a placeholder: nothing is stored through it
+  else if (!make_tmap_c(&th, H, (uint64_t)2 * F, (uint64_t)M, (uint64_t)ldh, false)) return FLB_ERR_TMA;
   return launch_pair<false, false, EPI_GATED_BF16>(ta, tb, th, 1, H, M, 2 * F, K, ldh, 0, st, stream, GroupArgs{nullptr, 0, 0}, 0, &tact, act_type);
 }
 
@@ -930,8 +965,8 @@ FLB_API int flb_gemm_gathered_bf16(const void* A, const void* B, void* C, int M,
   if (!ok) return FLB_ERR_TMA;
   if (!make_tmap_c(&tc, C, (uint64_t)N, (uint64_t)M, (uint64_t)ldc, false)) return FLB_ERR_TMA;
   GroupArgs group{nullptr, 0, 0, 0, arrive, arrive_target, chunk_rows, local_chunk};
-  const int num_m = (M + PairCfg::TILE_M - 1) / PairCfg::TILE_M;
-  group.m_rotate = (int)(((long long)local_chunk * chunk_rows / PairCfg::TILE_M) % num_m);
+  const int num_m = (M + PairTileM - 1) / PairTileM;
+  group.m_rotate = (int)(((long long)local_chunk * chunk_rows / PairTileM) % num_m);
   if (b_mn_major) return launch_pair<false, true, EPI_STORE_BF16, kGroupGathered>(ta, tb, tc, 1, C, M, N, K, ldc, 0, st, stream, group);
   return launch_pair<false, false, EPI_STORE_BF16, kGroupGathered>(ta, tb, tc, 1, C, M, N, K, ldc, 0, st, stream, group);
 }
@@ -953,8 +988,8 @@ FLB_API int flb_gemm_gathered_gated_bf16(const void* A, const void* W, void* H, 
   if (!make_tmap_c(&th, H, (uint64_t)2 * F, (uint64_t)M, (uint64_t)ldh, false)) return FLB_ERR_TMA;
   if (!make_tmap_c(&tact, ACT, (uint64_t)F, (uint64_t)M, (uint64_t)ldact, false)) return FLB_ERR_TMA;
   GroupArgs group{nullptr, 0, 0, 0, arrive, arrive_target, chunk_rows, local_chunk};
-  const int num_m = (M + PairCfg::TILE_M - 1) / PairCfg::TILE_M;
-  group.m_rotate = (int)(((long long)local_chunk * chunk_rows / PairCfg::TILE_M) % num_m);
+  const int num_m = (M + PairTileM - 1) / PairTileM;
+  group.m_rotate = (int)(((long long)local_chunk * chunk_rows / PairTileM) % num_m);
   return launch_pair<false, false, EPI_GATED_BF16, kGroupGathered>(ta, tb, th, 1, H, M, 2 * F, K, ldh, 0, st, stream, group, 0, &tact, act_type);
 }
 
@@ -975,7 +1010,7 @@ FLB_API int flb_gemm_scatter_maps(void* host_out, const void* const* dst_ptrs, i
 // CTA-pair launch over all rows, starting at row block `first_chunk * chunk_rows / 256`.
 FLB_API int flb_gemm_scatter_bf16(const void* A, const void* B, const void* scatter_maps, int M, int N, int K, long long lda, long long ldb,
                                   int b_mn_major, int chunk_rows, int first_chunk, cudaStream_t stream) {
-  if (M <= 0 || N <= 0 || K <= 0 || chunk_rows <= 0 || (chunk_rows % PairCfg::TILE_M) || scatter_maps == nullptr) return FLB_ERR_SHAPE;
+  if (M <= 0 || N <= 0 || K <= 0 || chunk_rows <= 0 || (chunk_rows % PairTileM) || scatter_maps == nullptr) return FLB_ERR_SHAPE;
   if ((lda % 8) || (ldb % 8) || (reinterpret_cast<uintptr_t>(scatter_maps) & 63)) return FLB_ERR_SHAPE;
   for (const void* ptr : {A, B})
     if (reinterpret_cast<uintptr_t>(ptr) & 15) return FLB_ERR_SHAPE;
@@ -989,8 +1024,8 @@ FLB_API int flb_gemm_scatter_bf16(const void* A, const void* B, const void* scat
   GroupArgs group{};
   group.scatter_maps = reinterpret_cast<const CUtensorMap*>(scatter_maps);
   group.scatter_chunk_rows = chunk_rows;
-  const int num_m = (M + PairCfg::TILE_M - 1) / PairCfg::TILE_M;
-  group.m_rotate = (int)(((long long)first_chunk * chunk_rows / PairCfg::TILE_M) % num_m);
+  const int num_m = (M + PairTileM - 1) / PairTileM;
+  group.m_rotate = (int)(((long long)first_chunk * chunk_rows / PairTileM) % num_m);
   // the kernel's own output map is unused in this mode: pass A's as a placeholder
   if (b_mn_major) return launch_pair<false, true, EPI_STORE_BF16, kGroupScatter>(ta, tb, ta, 1, nullptr, M, N, K, N, 0, st, stream, group);
   return launch_pair<false, false, EPI_STORE_BF16, kGroupScatter>(ta, tb, ta, 1, nullptr, M, N, K, N, 0, st, stream, group);

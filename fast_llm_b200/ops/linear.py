@@ -149,6 +149,9 @@ def linear(x, weight, bias=None, *, transposed_weight: bool = False, mode: str =
     """Differentiable linear layer; see the module docstring for `mode`."""
     # Flatten outside the autograd node so its output is a fresh tensor (rotary later rotates it in place).
     lead = x.shape[:-1]
+    if group is None and not torch.is_grad_enabled():
+        y = _forward_matmul(x.reshape(-1, x.shape[-1]), weight, transposed_weight)
+        return (y if bias is None else y + bias).view(*lead, y.shape[-1])
     y = _Linear.apply(x.reshape(-1, x.shape[-1]), weight, bias, transposed_weight, mode, group, sequence_parallel)
     if len(lead) != 1 and y.shape[0] == lead.numel():
         y = y.view(*lead, y.shape[-1])

@@ -177,4 +177,14 @@ _MLP._backward_fused = staticmethod(_backward_fused)
 
 def mlp(x, w1, b1, w2, b2, *, gated: bool, activation: ActivationType, group=None, sequence_parallel: bool = False,
         recompute_level: MLPRecomputeLevel = MLPRecomputeLevel.activation):
+    if group is None and not torch.is_grad_enabled():  # no backward pass: no node, nothing kept for it
+        x2 = x.reshape(-1, x.shape[-1])
+        if gated and b1 is None and gated_ok(x2, w1):
+            _, a = matmul_nt_gated(x2, w1, activation.code, keep_hidden=False)
+        else:
+            h = matmul_nt(x2, w1)
+            a = _act_fwd(h if b1 is None else h + b1, gated, activation)
+        y = matmul_nn(a, w2)
+        y = y if b2 is None else y + b2
+        return y.view(*x.shape[:-1], y.shape[-1])
     return _MLP.apply(x, w1, b1, w2, b2, gated, activation, group, sequence_parallel, recompute_level)

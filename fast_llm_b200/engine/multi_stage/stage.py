@@ -223,10 +223,7 @@ class Stage:
         assert self._mode.support_backward
         input_, output = context
         if output.requires_grad:
-            # On this thread: handing every stage's graph to the engine's device thread and back costs two thread wake-ups
-            # and a fight over the interpreter lock, and its nodes are Python anyway.
-            with torch.autograd.set_multithreading_enabled(False):
-                torch.autograd.backward(output, output_grad)
+            output.backward(output_grad)
         if torch.is_tensor(input_) and input_.is_floating_point() and input_.requires_grad:
             grad = input_.grad
             input_.grad = None

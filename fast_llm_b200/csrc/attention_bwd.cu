@@ -40,7 +40,7 @@ struct BwdParams {
   long long dkv_stride; // elements
   long long total_q, tok_groups;
   int heads, kv_heads, k_col0, v_col0, head_dim;
-  int kv_blocks_per_doc, splits;
+  int kv_blocks_per_doc;
   int causal, window;
   float scale, scale_log2;
   int* err_word;
@@ -70,13 +70,12 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int kv_head = blockIdx.y;
   const int group = p.heads / p.kv_heads;
-  const int rank = blockIdx.x % p.splits, block = blockIdx.x / p.splits;
-  const int doc = block / p.kv_blocks_per_doc;
-  const int jblk = block % p.kv_blocks_per_doc;
+  const int doc = blockIdx.x / p.kv_blocks_per_doc;
+  const int jblk = blockIdx.x % p.kv_blocks_per_doc;
   const int q_begin = p.cu_q[doc], q_len = p.cu_q[doc + 1] - q_begin;
   const int k_begin = p.cu_k[doc], k_len = p.cu_k[doc + 1] - k_begin;
   const int k0 = jblk * BN;
-  if (k0 >= k_len) return;  // uniform for the cluster
+  if (k0 >= k_len) return;
   const int shift = k_len - q_len;
   // query rows that can see keys [k0, k0 + BN): causal -> q >= k0 - shift; window -> q <= k0 + BN - 1 - shift + window - 1
   int q_lo = 0, q_hi = q_len;
@@ -84,9 +83,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
   if (p.window > 0) q_hi = min(q_len, k0 + BN - 1 - shift + p.window);
   const int iblk_lo = q_lo / BM, iblk_hi = (q_hi + BM - 1) / BM;
   const int blocks = max(iblk_hi - iblk_lo, 0);
-  // the CTAs of a cluster take turns at the pairs of this key block
-  const int all_pairs = blocks * group;
-  const int num_pairs = all_pairs > rank ? (all_pairs - rank + p.splits - 1) / p.splits : 0;
+  const int num_pairs = blocks * group;
 
   if (threadIdx.x == 0) {
     asm volatile("prefetch.tensormap [%0];" ::"l"(&tmap_q) : "memory");
@@ -110,8 +107,8 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
   auto tmem_t = [&](int i) { return tmem + 128u * (uint32_t)i; };
   const uint32_t tmem_dv = tmem + 256, tmem_dk = tmem + 384;
 
-  auto pair_head = [&](int n) { return kv_head * group + (rank + n * p.splits) / blocks; };
-  auto pair_q0 = [&](int n) { return (iblk_lo + (rank + n * p.splits) % blocks) * BM; };
+  auto pair_head = [&](int n) { return kv_head * group + n / blocks; };
+  auto pair_q0 = [&](int n) { return (iblk_lo + n % blocks) * BM; };
 
   if (warp == 0) {
     if (lane == 0) {
@@ -314,8 +311,6 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
       // the last commit (bar 9 of the last pair) covered every MMA; it was observed above
       tc_fence_after();
     }
-    // a CTA without a pair of its own: K and V must have landed before anything is written over them
-    if (p.splits > 1 && num_pairs == 0) mbar_wait(bar(0), 0, abort_flag, p.err_word, 52);
     const int krow = k0 + r;
     const bool have_acc = num_pairs > 0 && ok;  // warp-uniform
     __nv_bfloat16* base = p.dkv + (long long)(k_begin + min(krow, k_len - 1)) * p.dkv_stride + kv_head * p.head_dim + half * (HD / 2);
@@ -333,15 +328,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
 #pragma unroll
           for (int i = 0; i < 32; ++i) v[i] = 0u;
         }
-        if (p.splits > 1) {
-          // every MMA and copy of this CTA is complete: its operand tiles make room for the partial sums, [which][row][HD] fp32 with
-          // the 16-byte chunks of a row permuted so that the 32 rows of a warp spread over the banks
-          const int chunk0 = half * (HD / 8) + c * 8;
-#pragma unroll
-          for (int g = 0; g < 8; ++g)
-            *reinterpret_cast<uint4*>(smem + which * (128 * HD * 4) + r * (HD * 4) + (((chunk0 + g) ^ (r & 7)) << 4)) =
-                make_uint4(v[4 * g], v[4 * g + 1], v[4 * g + 2], v[4 * g + 3]);
-        } else if (krow < k_len) {
+        if (krow < k_len) {
 #pragma unroll
           for (int g = 0; g < 4; ++g) {
             if (half * (HD / 2) + c * 32 + g * 8 >= p.head_dim) break;
@@ -353,33 +340,6 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
         }
       }
     }
-  }
-
-  if (p.splits > 1) {
-    __syncthreads();
-    cluster_sync();
-    // each CTA adds up its share of the rows over the cluster, in rank order
-    const int rows = 128 / p.splits;
-    for (int i = threadIdx.x; i < 2 * rows * (HD / 8); i += kThreadsBwd) {
-      const int which = i / (rows * (HD / 8)), rest = i % (rows * (HD / 8));
-      const int row = rank * rows + rest / (HD / 8), c8 = rest % (HD / 8);
-      if (k0 + row >= k_len || c8 * 8 >= p.head_dim) continue;
-      float f[8];
-#pragma unroll
-      for (int e = 0; e < 8; ++e) f[e] = 0.f;
-      for (int q = 0; q < p.splits; ++q) {
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-          const uint32_t at = map_to_cta(sb + which * (128 * HD * 4) + row * (HD * 4) + (((2 * c8 + h) ^ (row & 7)) << 4), q);
-          float4 x;
-          asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(x.x), "=f"(x.y), "=f"(x.z), "=f"(x.w) : "r"(at) : "memory");
-          f[4 * h] += x.x; f[4 * h + 1] += x.y; f[4 * h + 2] += x.z; f[4 * h + 3] += x.w;
-        }
-      }
-      *reinterpret_cast<flb::bf16x8*>(p.dkv + (long long)(k_begin + k0 + row) * p.dkv_stride + kv_head * p.head_dim + (which == 0 ? p.k_col0 : p.v_col0) +
-                                      c8 * 8) = flb::pack8(f);
-    }
-    cluster_sync();  // nobody leaves while its sums are being read
   }
 
   tc_fence_before();
@@ -528,31 +488,10 @@ FLB_API int flb_attention_bwd(const void* q, long long q_stride, int q_col0, con
   p.causal = causal; p.window = window; p.scale = softmax_scale; p.scale_log2 = softmax_scale * 1.4426950408889634f;
   p.err_word = bwd_err_word();
   if (!p.err_word) return FLB_ERR_CUDA;
-  // A key block walks all its (query head, query block) pairs one after the other, so a long document is a long chain on few SMs: a
-  // cluster of up to four CTAs shares the pairs of a block and adds up dK and dV over distributed shared memory.  A CTA costs about
-  // five pairs to set up, so where the SMs are taken already (up to four CTAs each: they differ in length by the position of their
-  // block) every CTA keeps four pairs on average; idle SMs are filled in any case.  Eight layers at 4096 tokens, 16 / 4 heads of 64,
-  // five documents: 1.71 -> 1.16 ms; 8192 tokens, 32 / 8 heads of 128, two documents: 1.77 -> 1.6 ms a layer.
-  const long long blocks = (total_k + BN - 1) / BN * kv_heads;
-  const int group = heads / kv_heads, longest = p.kv_blocks_per_doc * group;
-  const long long average = group * ((total_k / batch + BN - 1) / BN + 1) / 2;  // pairs of a block, causal
-  p.splits = 1;
-  while (p.splits < 4 && longest >= 4 * p.splits &&
-         (blocks * p.splits * 2 <= 148 || (blocks * p.splits < 4 * 148 && average >= 8 * p.splits)))
-    p.splits *= 2;
-  cudaLaunchConfig_t config{};
-  config.gridDim = dim3(p.kv_blocks_per_doc * batch * p.splits, kv_heads);
-  config.blockDim = dim3(kThreadsBwd);
-  config.dynamicSmemBytes = wide ? Bwd<128>::TOTAL : Bwd<64>::TOTAL;
-  config.stream = stream;
-  cudaLaunchAttribute cluster;
-  cluster.id = cudaLaunchAttributeClusterDimension;
-  cluster.val.clusterDim.x = p.splits;
-  cluster.val.clusterDim.y = cluster.val.clusterDim.z = 1;
-  config.attrs = &cluster;
-  config.numAttrs = 1;
-  e = wide ? cudaLaunchKernelEx(&config, attn_bwd_kernel<128>, tq, tk, tv, tdo, p) : cudaLaunchKernelEx(&config, attn_bwd_kernel<64>, tq, tk, tv, tdo, p);
-  if (e != cudaSuccess) return flb_record_cuda_error(e);
+  dim3 grid(p.kv_blocks_per_doc * batch, kv_heads);
+  if (wide) attn_bwd_kernel<128><<<grid, kThreadsBwd, Bwd<128>::TOTAL, stream>>>(tq, tk, tv, tdo, p);
+  else attn_bwd_kernel<64><<<grid, kThreadsBwd, Bwd<64>::TOTAL, stream>>>(tq, tk, tv, tdo, p);
+  FLB_CHECK_LAUNCH();
   if (wide) attn_dq_convert_kernel<128><<<148 * 8, 256, 0, stream>>>(dq_accum, (__nv_bfloat16*)dq, dq_stride, q_col0, total_q, tok_groups, heads, head_dim);
   else attn_dq_convert_kernel<64><<<148 * 8, 256, 0, stream>>>(dq_accum, (__nv_bfloat16*)dq, dq_stride, q_col0, total_q, tok_groups, heads, head_dim);
   FLB_CHECK_LAUNCH();

@@ -937,27 +937,3 @@ def test_packed_attention_head_sizes(doc_lengths, heads, kv_heads, d, window):
     # P and dS enter the second product rounded to bf16, as in the 128-wide cases above
     assert _rel_err(out, ref) < 1.5e-2
     assert torch.isfinite(qkv.grad).all() and _rel_err(qkv.grad, x.grad) < 2e-2
-
-
-@pytest.mark.parametrize("doc_lengths, heads, kv_heads, d", [
-    ([1300], 4, 1, 64),  # one key/value head: clusters of four, the last key blocks with fewer pairs than CTAs
-    ([100, 3], 1, 1, 128),  # a single pair
-    ([2000, 700], 8, 2, 128),
-])
-def test_attention_backward_shared_between_the_ctas_of_a_cluster(doc_lengths, heads, kv_heads, d):
-    """Few key blocks: the pairs of a block are shared by a cluster, dK and dV are summed over its CTAs."""
-    from fast_llm_b200.ops import _lib
-    from fast_llm_b200.ops.attention import attention_reference, packed_attention
-
-    torch.manual_seed(5)
-    total, nq, nkv = sum(doc_lengths), heads * d, kv_heads * d
-    qkv = torch.randn(total, nq + 2 * nkv, device="cuda", dtype=torch.bfloat16, requires_grad=True)
-    cu = torch.tensor([0] + list(torch.tensor(doc_lengths).cumsum(0)), device="cuda", dtype=torch.int32)
-    g = torch.randn(total, nq, device="cuda", dtype=torch.bfloat16)
-    packed_attention(qkv, cu, max(doc_lengths), heads, kv_heads, d).backward(g)
-    assert _lib.get_lib().flb_attention_bwd_error_word() == 0
-    x = qkv.detach().float().requires_grad_()
-    attention_reference(x[:, :nq].reshape(total, heads, d), x[:, nq : nq + nkv].reshape(total, kv_heads, d), x[:, nq + nkv :].reshape(total, kv_heads, d), cu,
-                        cu, True, None, d**-0.5).reshape(total, nq).backward(g.float())
-    for name, lo, hi in (("dq", 0, nq), ("dk", nq, nq + nkv), ("dv", nq + nkv, nq + 2 * nkv)):
-        assert _rel_err(qkv.grad[:, lo:hi], x.grad[:, lo:hi]) < 3e-2, name

@@ -139,15 +139,6 @@ def stream_ptr() -> int:
     return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
 
 
-class KernelFunction(torch.autograd.Function):
-    """`autograd.Function` for the hand-written nodes.  The stock `apply` inspects the arguments for functorch wrappers in Python
-    (about 5 us per node); these nodes call raw kernels and cannot run under functorch transforms anyway."""
-
-    @classmethod
-    def apply(cls, *args):
-        return super(torch.autograd.Function, cls).apply(*args)
-
-
 def ptr(t: "torch.Tensor | None") -> int | None:
     return None if t is None else t.data_ptr()
 

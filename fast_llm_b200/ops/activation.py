@@ -9,7 +9,6 @@ import enum
 import torch
 
 from fast_llm_b200.ops import _lib
-from fast_llm_b200.ops._lib import KernelFunction
 
 
 class ActivationType(str, enum.Enum):
@@ -84,7 +83,7 @@ def act_bwd_native(grad_out2, x2, gated: bool, act: ActivationType, recompute: b
     return grad_in, out
 
 
-class _MLPActivation(KernelFunction):
+class _MLPActivation(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x, gated, act):
         shape = x.shape

@@ -15,7 +15,6 @@ attention.py:209-256`).
 import torch
 
 from fast_llm_b200.ops import _lib
-from fast_llm_b200.ops._lib import KernelFunction
 
 
 def attention_reference(q, k, v, cu_seqlens_q, cu_seqlens_k, causal: bool, window_size: int | None, scale: float):
@@ -99,7 +98,7 @@ def _joint_key_value_rows(k: torch.Tensor, v: torch.Tensor) -> torch.Tensor:
     return torch.cat([k.reshape(tk, width), v.reshape(tk, width)], dim=1)
 
 
-class _NativeAttention(KernelFunction):
+class _NativeAttention(torch.autograd.Function):
     """q [Tq, heads, d], k / v [Tk, kv_heads, d]; the key segments may be longer than the query segments (a prefix from
     earlier micro-sequences or other sequence-data ranks): masks are bottom-right aligned."""
 
@@ -131,7 +130,7 @@ class _NativeAttention(KernelFunction):
         return dq.view(tq, heads, d), dkv[:, :width].view(tk, kv_heads, d), dkv[:, width:].view(tk, kv_heads, d), None, None, None, None, None, None, None
 
 
-class _PackedNativeAttention(KernelFunction):
+class _PackedNativeAttention(torch.autograd.Function):
     """Self-attention over the fused projection output [tokens, (heads + 2 kv_heads) x d]; the backward writes dq, dk and
     dv into one packed gradient, so the projection's backward is one GEMM."""
 

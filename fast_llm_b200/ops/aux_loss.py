@@ -5,10 +5,8 @@ Parity: `fast_llm/functional/utils.py:63-80` (AuxiliaryLoss).
 
 import torch
 
-from fast_llm_b200.ops._lib import KernelFunction
 
-
-class _AuxiliaryLoss(KernelFunction):
+class _AuxiliaryLoss(torch.autograd.Function):
     @staticmethod
     def forward(ctx, activation, loss, grad_scale):
         ctx.grad = torch.full_like(loss, grad_scale) if not torch.is_tensor(grad_scale) else grad_scale.to(loss.dtype).reshape(loss.shape)

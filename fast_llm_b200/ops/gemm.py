@@ -17,9 +17,8 @@ from fast_llm_b200.ops import _lib
 _EPI_STORE_BF16, _EPI_STORE_F32, _EPI_ACC_F32, _EPI_ACC_BF16 = 0, 1, 2, 3
 
 
-# Read once: an environment lookup per GEMM is 2 us of host time, as much as the launch itself.
-_BACKEND = os.environ.get("FLB_GEMM", "tcgen05")
-_BLOCK_N = int(os.environ.get("FLB_GEMM_BLOCK_N", 0))
+def _backend() -> str:
+    return os.environ.get("FLB_GEMM", "tcgen05")
 
 
 def _native_ok(a: torch.Tensor, b: torch.Tensor) -> bool:
@@ -27,7 +26,7 @@ def _native_ok(a: torch.Tensor, b: torch.Tensor) -> bool:
         a.is_cuda
         and a.dtype == torch.bfloat16
         and b.dtype == torch.bfloat16
-        and _BACKEND == "tcgen05"
+        and _backend() == "tcgen05"
         and a.stride(-1) == 1
         and b.stride(-1) == 1
         and a.stride(0) % 8 == 0
@@ -44,8 +43,8 @@ def _note_library_fallback(a: torch.Tensor, b: torch.Tensor, out: torch.Tensor) 
     """A CUDA GEMM that the tcgen05 kernels do not take is counted and announced once per reason: nothing falls back silently."""
     if not a.is_cuda:
         return
-    if _BACKEND != "tcgen05":
-        reason = f"FLB_GEMM={_BACKEND}"
+    if _backend() != "tcgen05":
+        reason = f"FLB_GEMM={_backend()}"
     elif a.dtype != torch.bfloat16 or b.dtype != torch.bfloat16:
         reason = f"operand dtypes {a.dtype}, {b.dtype} (the tcgen05 kernels take bf16)"
     elif a.stride(-1) != 1 or b.stride(-1) != 1 or out.stride(-1) != 1:
@@ -70,7 +69,7 @@ def gemm_raw(a, b, out, m, n, k, a_mn, b_mn, epilogue, block_n=None, max_ctas=0,
     tensor-parallel peer's symmetric memory); `direct_store` writes C with register stores instead of TMA."""
     lib = _lib.get_lib()
     if block_n is None:
-        block_n = _BLOCK_N
+        block_n = int(os.environ.get("FLB_GEMM_BLOCK_N", 0))
     _lib.check(
         lib.flb_gemm_bf16_ex(
             a.data_ptr() if a_ptr is None else a_ptr, b.data_ptr() if b_ptr is None else b_ptr,

@@ -11,7 +11,6 @@ matmuls), `fast_llm/functional/triton/mlp.py:207-477` (`mlp_autograd` with a spa
 import torch
 
 from fast_llm_b200.ops import _lib
-from fast_llm_b200.ops._lib import KernelFunction
 from fast_llm_b200.ops.activation import ActivationType, act_bwd_native, mlp_activation
 from fast_llm_b200.ops.gemm import _EPI_STORE_BF16, _epilogue
 from fast_llm_b200.ops.param_grad import wgrad_target
@@ -59,7 +58,7 @@ def grouped_wgrad(a: torch.Tensor, b: torch.Tensor, out: torch.Tensor, row_begin
     return out
 
 
-class _GroupedMLP(KernelFunction):
+class _GroupedMLP(torch.autograd.Function):
     """y = act(x W1_e^T) W2_e for the expert e owning each row; W1 [experts * (1 + gated) * ffn, hidden], W2 [experts * ffn, hidden]."""
 
     @staticmethod
@@ -126,7 +125,7 @@ def _combine_raw(y, rows, scores) -> torch.Tensor:
     return out
 
 
-class _Dispatch(KernelFunction):
+class _Dispatch(torch.autograd.Function):
     """xs[rows[t, j]] = x[t]: copies every token to the row of each of its experts."""
 
     @staticmethod
@@ -140,7 +139,7 @@ class _Dispatch(KernelFunction):
         return _combine_raw(grad.contiguous(), rows, None), None, None
 
 
-class _Combine(KernelFunction):
+class _Combine(torch.autograd.Function):
     """out[t] = sum_j scores[t, j] * y[rows[t, j]]"""
 
     @staticmethod

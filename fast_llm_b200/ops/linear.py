@@ -12,7 +12,6 @@ epilogue straight into the parameter's gradient buffer.  Parity: `fast_llm/funct
 
 import torch
 
-from fast_llm_b200.ops._lib import KernelFunction
 from fast_llm_b200.ops.gemm import matmul_nn, matmul_nt, matmul_tn
 from fast_llm_b200.ops.param_grad import accumulate_param_grad, wgrad_target
 from fast_llm_b200.parallel import fused_tp
@@ -48,7 +47,7 @@ def bias_grad(dy2: torch.Tensor, bias: torch.Tensor):
     return accumulate_param_grad(bias, dy2.sum(0, dtype=torch.float32).to(bias.dtype) if dy2.dtype != torch.float32 else dy2.sum(0))
 
 
-class _Linear(KernelFunction):
+class _Linear(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x, weight, bias, transposed_weight, mode, group, sequence_parallel):
         shape = x.shape
@@ -149,9 +148,6 @@ def linear(x, weight, bias=None, *, transposed_weight: bool = False, mode: str =
     """Differentiable linear layer; see the module docstring for `mode`."""
     # Flatten outside the autograd node so its output is a fresh tensor (rotary later rotates it in place).
     lead = x.shape[:-1]
-    if group is None and not torch.is_grad_enabled():
-        y = _forward_matmul(x.reshape(-1, x.shape[-1]), weight, transposed_weight)
-        return (y if bias is None else y + bias).view(*lead, y.shape[-1])
     y = _Linear.apply(x.reshape(-1, x.shape[-1]), weight, bias, transposed_weight, mode, group, sequence_parallel)
     if len(lead) != 1 and y.shape[0] == lead.numel():
         y = y.view(*lead, y.shape[-1])

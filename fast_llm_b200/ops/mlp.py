@@ -15,7 +15,6 @@ import enum
 
 import torch
 
-from fast_llm_b200.ops._lib import KernelFunction
 from fast_llm_b200.ops.activation import ActivationType, _native as _act_native, act_bwd_native, act_fwd_native, mlp_activation_reference
 from fast_llm_b200.ops.gemm import gated_ok, matmul_nn, matmul_nt, matmul_nt_gated
 from fast_llm_b200.ops.linear import bias_grad, needs_weight_grad, weight_grad
@@ -58,9 +57,9 @@ def _act_bwd(da, h, gated, act, recompute):
     return dh, (a.detach() if recompute else None)
 
 
-class _MLP(KernelFunction):
+class _MLP(torch.autograd.Function):
     @staticmethod
-    def forward(ctx, x, w1, b1, w2, b2, gated, act, group, sequence_parallel, recompute):
+    def forward(ctx, x, w1, b1, w2, b2, gated, act, group, sequence_parallel, recompute, keep_hidden):
         shape = x.shape
         x_in = x.reshape(-1, shape[-1])
         fused = _fused_context(x_in, w1, b1, w2, b2, group, sequence_parallel)
@@ -81,7 +80,7 @@ class _MLP(KernelFunction):
         ctx.fused = None
         x2 = gather_op(x_in, group, 0) if (sequence_parallel and group is not None) else x_in
         if gated and b1 is None and gated_ok(x2, w1):
-            h, a = matmul_nt_gated(x2, w1, act.code)  # the activation rides in the GEMM's epilogue
+            h, a = matmul_nt_gated(x2, w1, act.code, keep_hidden)  # the activation rides in the GEMM's epilogue
         else:
             h = matmul_nt(x2, w1)
             if b1 is not None:
@@ -132,7 +131,7 @@ class _MLP(KernelFunction):
             handle.wait()
         if dx is not None and dx.numel() == x_saved.numel() and len(shape) != 2:
             dx = dx.view(shape)
-        return dx, dw1, db1, dw2, db2, None, None, None, None, None
+        return dx, dw1, db1, dw2, db2, None, None, None, None, None, None
 
 
 def _fused_context(x_in, w1, b1, w2, b2, group, sequence_parallel):
@@ -169,7 +168,7 @@ def _backward_fused(ctx, dy2, x_saved, h, a):
     dw1 = weight_grad(dh, fused.finish_gather(pending_x), w1, transposed_weight=False)
     if dx is not None and len(shape) != 2:
         dx = dx.view(shape)
-    return dx, dw1, None, dw2, None, None, None, None, None, None
+    return dx, dw1, None, dw2, None, None, None, None, None, None, None
 
 
 _MLP._backward_fused = staticmethod(_backward_fused)
@@ -177,14 +176,5 @@ _MLP._backward_fused = staticmethod(_backward_fused)
 
 def mlp(x, w1, b1, w2, b2, *, gated: bool, activation: ActivationType, group=None, sequence_parallel: bool = False,
         recompute_level: MLPRecomputeLevel = MLPRecomputeLevel.activation):
-    if group is None and not torch.is_grad_enabled():  # no backward pass: no node, nothing kept for it
-        x2 = x.reshape(-1, x.shape[-1])
-        if gated and b1 is None and gated_ok(x2, w1):
-            _, a = matmul_nt_gated(x2, w1, activation.code, keep_hidden=False)
-        else:
-            h = matmul_nt(x2, w1)
-            a = _act_fwd(h if b1 is None else h + b1, gated, activation)
-        y = matmul_nn(a, w2)
-        y = y if b2 is None else y + b2
-        return y.view(*x.shape[:-1], y.shape[-1])
-    return _MLP.apply(x, w1, b1, w2, b2, gated, activation, group, sequence_parallel, recompute_level)
+    # without a backward pass the first layer's output need not reach memory
+    return _MLP.apply(x, w1, b1, w2, b2, gated, activation, group, sequence_parallel, recompute_level, torch.is_grad_enabled())

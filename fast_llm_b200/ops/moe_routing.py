@@ -12,7 +12,6 @@ Parity: `fast_llm/layers/decoder/mlp/mixture_of_experts.py:237-262`, `fast_llm/f
 import torch
 
 from fast_llm_b200.ops import _lib
-from fast_llm_b200.ops._lib import KernelFunction
 
 MAX_EXPERTS, MAX_TOP_K = 64, 8
 
@@ -21,7 +20,7 @@ def native_routing_available(logits: torch.Tensor, k: int) -> bool:
     return logits.is_cuda and logits.dtype == torch.float32 and logits.dim() == 2 and logits.shape[1] <= MAX_EXPERTS and k <= MAX_TOP_K
 
 
-class _RouteTopK(KernelFunction):
+class _RouteTopK(torch.autograd.Function):
     @staticmethod
     def forward(ctx, logits, k, aux_weight, z_weight):
         logits = logits.contiguous()

@@ -8,7 +8,6 @@ gradients accumulated into the gradient buffer.
 import torch
 
 from fast_llm_b200.ops import _lib
-from fast_llm_b200.ops._lib import KernelFunction
 from fast_llm_b200.ops.param_grad import accumulate_param_grad, has_grad_buffer
 
 
@@ -85,7 +84,7 @@ def _reduce_param_grad(param, partial):
     return out.to(param.dtype)
 
 
-class _NormFunction(KernelFunction):
+class _NormFunction(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x, delta, weight, bias, eps, zero_centered, layer_norm):
         shape = x.shape

@@ -7,7 +7,6 @@ helpers (`fast_llm/layers/language_model/embedding.py:74`, `fast_llm/layers/deco
 import torch
 
 from fast_llm_b200.ops import _lib
-from fast_llm_b200.ops._lib import KernelFunction
 
 _DT = {torch.float32: 0, torch.bfloat16: 1}
 
@@ -59,7 +58,7 @@ def bias_residual(x: torch.Tensor, bias: torch.Tensor | None, residual: torch.Te
     return out if residual is None else out + residual
 
 
-class _Embedding(KernelFunction):
+class _Embedding(torch.autograd.Function):
     @staticmethod
     def forward(ctx, ids, weight, vocab_begin, vocab_end, scale):
         from fast_llm_b200.ops.param_grad import has_grad_buffer

@@ -8,7 +8,6 @@ kernel.  Pairing is element i with i + rot_dim/2 inside a head, the "real/imagin
 import torch
 
 from fast_llm_b200.ops import _lib
-from fast_llm_b200.ops._lib import KernelFunction
 
 
 def rope_reference(x: torch.Tensor, table: torch.Tensor, positions: torch.Tensor | None, n_heads: int, head_dim: int,
@@ -46,7 +45,7 @@ def rope_(x: torch.Tensor, table: torch.Tensor, positions: torch.Tensor | None, 
     return x
 
 
-class _Rope(KernelFunction):
+class _Rope(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x, table, positions, n_heads, head_dim, rot_dim):
         ctx.save_for_backward(table, positions)

@@ -17,8 +17,6 @@ import typing
 
 import torch
 
-from fast_llm_b200.ops._lib import KernelFunction
-
 
 # ----------------------------------------------------------------------------------------------------------------------
 # chunk loop with boundary-state checkpointing
@@ -122,7 +120,7 @@ def causal_conv1d_reference(x, weight, bias, document_index, activation) -> torc
     return activation_reference(out, activation).to(x.dtype)
 
 
-class _CausalConv1d(KernelFunction):
+class _CausalConv1d(torch.autograd.Function):
     TOKENS_PER_BLOCK = 64
 
     @staticmethod
@@ -202,7 +200,7 @@ def _selective_scan_step(state, chunk_in, shared):
     return y.to(x.dtype), states[-1]
 
 
-class _SelectiveScan(KernelFunction):
+class _SelectiveScan(torch.autograd.Function):
     """Chunk-parallel CUDA scan (`csrc/ssm.cu`): three launches forward, four backward; the only saved state beyond the
     inputs is the [chunks, state, channels] start state and decay product of every 64-token chunk."""
 
@@ -339,7 +337,7 @@ def _chunk_layout(boundaries: list[int], chunk: int, device):
     return index.to(device), first
 
 
-class _DeltaStateScan(KernelFunction):
+class _DeltaStateScan(torch.autograd.Function):
     """State entering every chunk of S_{c+1} = decay_c o S_c - mix_c S_c + write_c (zero at document starts): one CUDA kernel
     walks the chunks (`flb_delta_state_scan`), a second one the adjoint recurrence; the gradients of mix, write and decay are
     batched products of the two results."""
@@ -447,7 +445,7 @@ def _delta_rule_all_chunks(q, k, v, g, beta, boundaries: list[int], chunk: int) 
     return out.transpose(1, 2)[valid].to(out_dtype)
 
 
-class _DeltaRule(KernelFunction):
+class _DeltaRule(torch.autograd.Function):
     """The delta rule in five kernels (`csrc/delta.cu`): per chunk of 64 tokens the triangular system and its inverse, a scan over
     the chunks of every document for the states, the outputs; backward, the adjoint scan and the gradients chunk by chunk.
     q, k may have fewer heads than v (each serves that many adjacent value heads) and any row stride."""

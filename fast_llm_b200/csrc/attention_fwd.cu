@@ -372,6 +372,7 @@ template <int HD>
 __global__ void __launch_bounds__(kThreadsAttn, 1)
 attn_fwd_kernel_v2(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k, const __grid_constant__ CUtensorMap tmap_v,
                    const AttnParams p) {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");  // a dependent only reads weights before it waits for this kernel
   using C = Fwd2<HD>;
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw_addr = smem_u32(smem_raw);

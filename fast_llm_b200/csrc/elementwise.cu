@@ -57,6 +57,7 @@ __global__ void rope_kernel(__nv_bfloat16* __restrict__ x, const float* __restri
 // in: [rows, (gated?2:1)*n] (gate columns first, then up columns); out: [rows, n]
 __global__ void act_fwd_kernel(const __nv_bfloat16* __restrict__ in, __nv_bfloat16* __restrict__ out, long long rows,
                                int n, int gated, int type) {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");  // a dependent only reads weights before it waits for this kernel
   const int nvec = n >> 3;
   const long long total = rows * nvec;
   const long long in_stride = gated ? 2ll * n : n;

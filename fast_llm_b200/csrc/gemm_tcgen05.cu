@@ -218,6 +218,117 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
 }
 
 // ------------------------------------------------------------------------------------------------
+// Few rows (up to 32, a generation step): one narrow tile per CTA
+// ------------------------------------------------------------------------------------------------
+// Bounded by the weights' trip from HBM: 256-wide tiles leave a 3072-wide projection on 12 SMs with 128 KB in flight in all.  Tiles
+// of 32 columns (64 where B is N-major or there are enough of them for the chip) and deep rings put every SM to work.  Of the 128
+// rows of A that the MMA reads only 32 are copied: the rest is whatever shared memory holds (later stages, B), its accumulator
+// rows are never read.  The MMAs of an output element are those of the wide tiles in the same order, so the results are the same
+// bits.  8 blocks of 2048 / 8192, 24 steps of one row after a prompt of 100 and of 8 rows after 512: see flb_decode_step.
+constexpr int kFewRows = 32;
+template <int BLOCK_N>
+struct RowsCfg {
+  static constexpr int A_BYTES = kFewRows * BLOCK_K * 2, B_BYTES = BLOCK_N * BLOCK_K * 2;
+  static constexpr int STAGES = BLOCK_N == 32 ? 12 : 16;
+  static constexpr int B_OFFSET = STAGES * A_BYTES, BARS = B_OFFSET + STAGES * B_BYTES;
+  static constexpr int SMEM_BYTES = BARS + 512 + 1024;
+  static_assert((STAGES - 1) * A_BYTES + BLOCK_M * BLOCK_K * 2 <= BARS, "the MMA's 128 rows stay inside the allocation");
+};
+
+template <int BLOCK_N, bool B_MN, int EPI>
+__global__ void __launch_bounds__(96)
+gemm_rows_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b, void* __restrict__ Cv, int M, int N, int K,
+                 long long ldc, int* __restrict__ err_word) {
+  using C = RowsCfg<BLOCK_N>;
+  extern __shared__ uint8_t smem_raw[];
+  const uint32_t raw_addr = smem_u32(smem_raw);
+  const uint32_t pad = (1024u - (raw_addr & 1023u)) & 1023u;
+  const uint32_t base = raw_addr + pad, bars = base + C::BARS;
+  auto full_bar = [&](int s) { return bars + 8u * s; };
+  auto empty_bar = [&](int s) { return bars + 8u * (C::STAGES + s); };
+  const uint32_t done_bar = bars + 8u * (2 * C::STAGES);
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem_raw + pad + C::BARS + 8 * (2 * C::STAGES + 1));
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < C::STAGES; ++s) {
+      mbar_init(full_bar(s), 1);
+      mbar_init(empty_bar(s), 1);
+    }
+    mbar_init(done_bar, 1);
+    *abort_flag = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+  }
+  if (warp == 0) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"((uint32_t)BLOCK_N) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem = *tmem_slot;
+  const int n0 = blockIdx.x * BLOCK_N, num_kb = (K + BLOCK_K - 1) / BLOCK_K;
+
+  if (warp == 1) {
+    if (lane == 0) {
+      auto load_b = [&](int kb, int s) {
+        mbar_expect_tx(full_bar(s), C::A_BYTES + C::B_BYTES);
+        if constexpr (!B_MN) tma_load_2d(base + C::B_OFFSET + s * C::B_BYTES, &tmap_b, full_bar(s), kb * BLOCK_K, n0);
+        else tma_load_2d(base + C::B_OFFSET + s * C::B_BYTES, &tmap_b, full_bar(s), n0, kb * BLOCK_K);
+      };
+      auto load_a = [&](int kb, int s) { tma_load_2d(base + s * C::A_BYTES, &tmap_a, full_bar(s), kb * BLOCK_K, 0); };
+      // weights do not depend on the kernel before this one
+      const int ahead = min(num_kb, C::STAGES);
+      for (int kb = 0; kb < ahead; ++kb) load_b(kb, kb);
+      asm volatile("griddepcontrol.wait;" ::: "memory");
+      for (int kb = 0; kb < ahead; ++kb) load_a(kb, kb);
+      bool ok = true;
+      for (int kb = ahead; kb < num_kb && ok; ++kb) {
+        const int s = kb % C::STAGES;
+        if (!mbar_wait(empty_bar(s), ((kb / C::STAGES) & 1) ^ 1u, abort_flag, err_word, 11)) { ok = false; break; }
+        load_b(kb, s);
+        load_a(kb, s);
+      }
+      if (!ok) {  // copies already issued get a bounded chance to land before the CTA exits
+        const long long t0 = clock64();
+        while (clock64() - t0 < 2000000ll) {}
+      }
+    }
+  } else if (warp == 2) {
+    if (lane == 0) {
+      constexpr uint32_t idesc = make_idesc(BLOCK_M, BLOCK_N, false, B_MN);
+      bool ok = true;
+      for (int kb = 0; kb < num_kb; ++kb) {
+        const int s = kb % C::STAGES;
+        if (!mbar_wait(full_bar(s), (kb / C::STAGES) & 1, abort_flag, err_word, 12)) { ok = false; break; }
+        tc_fence_after();
+        const uint64_t adesc = make_smem_desc(base + s * C::A_BYTES, 16, 1024);
+        const uint32_t b_addr = base + C::B_OFFSET + s * C::B_BYTES;
+        const uint64_t bdesc = B_MN ? make_smem_desc(b_addr, 8192, 1024) : make_smem_desc(b_addr, 16, 1024);
+#pragma unroll
+        for (int k = 0; k < BLOCK_K / UMMA_K; ++k)
+          umma_bf16(tmem, adesc + (uint64_t)(k * 32 >> 4), bdesc + (uint64_t)(B_MN ? (k * 2048 >> 4) : (k * 32 >> 4)), idesc, (kb | k) != 0 ? 1u : 0u);
+        umma_commit(empty_bar(s));
+      }
+      if (ok) umma_commit(done_bar);
+    }
+  } else if (mbar_wait(done_bar, 0, abort_flag, err_word, 13)) {
+    tc_fence_after();
+#pragma unroll
+    for (int c = 0; c < BLOCK_N / 32; ++c) {
+      uint32_t r[32];
+      tmem_ld32(tmem + c * 32, r);
+      tmem_wait_ld();
+      store_chunk<EPI>(r, Cv, lane, n0 + c * 32, M, N, ldc);
+    }
+  }
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"((uint32_t)BLOCK_N) : "memory");
+}
+
+// ------------------------------------------------------------------------------------------------
 // CTA-pair kernel: clusters of two CTAs, 256 x 256 tiles, tcgen05.mma.cta_group::2 issued by the leader (cluster rank 0)
 // ------------------------------------------------------------------------------------------------
 constexpr int PairTileM = 256, PairTileN = 256;
@@ -757,6 +868,44 @@ int launch(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& tc, 
   return FLB_OK;
 }
 
+template <int BLOCK_N, bool B_MN, int EPI>
+int launch_rows(const CUtensorMap& ta, const CUtensorMap& tb, void* C, int M, int N, int K, long long ldc, bool overlap, DeviceState* st, cudaStream_t stream) {
+  using Cf = RowsCfg<BLOCK_N>;
+  auto kern = gemm_rows_kernel<BLOCK_N, B_MN, EPI>;
+  static const cudaError_t ready = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Cf::SMEM_BYTES);
+  if (ready != cudaSuccess) return flb_record_cuda_error(ready);
+  cudaLaunchConfig_t config{};
+  config.gridDim = dim3((N + BLOCK_N - 1) / BLOCK_N);
+  config.blockDim = dim3(96);
+  config.dynamicSmemBytes = Cf::SMEM_BYTES;
+  config.stream = stream;
+  cudaLaunchAttribute attribute;
+  attribute.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attribute.val.programmaticStreamSerializationAllowed = 1;
+  config.attrs = &attribute;
+  config.numAttrs = overlap ? 1 : 0;
+  const cudaError_t e = cudaLaunchKernelEx(&config, kern, ta, tb, C, M, N, K, ldc, st->err_word);
+  return e == cudaSuccess ? FLB_OK : flb_record_cuda_error(e);
+}
+
+// Up to 32 rows: see gemm_rows_kernel.
+int gemm_rows(const void* A, const void* B, void* C, int M, int N, int K, long long lda, long long ldb, long long ldc, bool b_mn, int epilogue,
+              bool overlap, DeviceState* st, cudaStream_t stream) {
+  // 32-wide tiles until two waves of 64-wide ones fill the chip; an N-major panel is 64 columns
+  const bool narrow = !b_mn && N <= 2 * 64 * st->num_sms;
+  CUtensorMap ta, tb;
+  if (!make_tmap(&ta, A, (uint64_t)K, (uint64_t)M, (uint64_t)lda, BLOCK_K, kFewRows)) return FLB_ERR_TMA;
+  if (!(b_mn ? make_tmap(&tb, B, (uint64_t)N, (uint64_t)K, (uint64_t)ldb, 64, BLOCK_K)
+             : make_tmap(&tb, B, (uint64_t)K, (uint64_t)N, (uint64_t)ldb, BLOCK_K, narrow ? 32 : 64))) return FLB_ERR_TMA;
+#define FLB_ROWS(BN, MN)                                                                                                             \
+  return epilogue == EPI_STORE_F32 ? launch_rows<BN, MN, EPI_STORE_F32>(ta, tb, C, M, N, K, ldc, overlap, st, stream)               \
+                                   : launch_rows<BN, MN, EPI_STORE_BF16>(ta, tb, C, M, N, K, ldc, overlap, st, stream)
+  if (b_mn) FLB_ROWS(64, true);
+  if (narrow) FLB_ROWS(32, false);
+  FLB_ROWS(64, false);
+#undef FLB_ROWS
+}
+
 template <bool A_MN, bool B_MN, int EPI, int GROUP = kGroupNone>
 int launch_pair(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& tc, int use_tc, void* C, int M, int N, int K,
                 long long ldc, int max_ctas, DeviceState* st, cudaStream_t stream, GroupArgs group = GroupArgs{nullptr, 0, 0},
@@ -815,10 +964,11 @@ int dispatch_major(int a_mn, int b_mn, int epi, const CUtensorMap& ta, const CUt
 //   a_mn_major = 0: A stored [M][lda] (K contiguous); 1: A stored [K][lda] (M contiguous).
 //   b_mn_major = 0: B stored [N][ldb] (K contiguous); 1: B stored [K][ldb] (N contiguous).
 //   epilogue: 0 store bf16, 1 store fp32, 2 C(fp32) += D, 3 C(bf16) += D.   ldc in elements of C.
-//   block_n: 0 = choose; 128 / 256 = one-CTA kernel with that tile width; 512 = CTA-pair kernel (256 x 256 tiles).
+//   block_n: 0 = choose (up to 32 rows of a K-major A: gemm_rows_kernel); 128 / 256 = one-CTA kernel with that tile width; 512 = CTA-pair kernel (256 x 256 tiles).
 //   max_ctas: limit the persistent grid (0 = one CTA per SM).
 // Pointers must be 16-byte aligned and lda/ldb multiples of 8 elements (TMA stride rule).
-// flags: bit 0 = write C with plain register stores instead of TMA (used when C is another GPU's memory).
+// flags: bit 0 = write C with plain register stores instead of TMA (used when C is another GPU's memory); bit 1 = up to 32 rows: may
+// start reading B before the kernel ahead of it in the stream has finished (which then must not write B).
 FLB_API int flb_gemm_bf16_ex(const void* A, const void* B, void* C, int M, int N, int K, long long lda, long long ldb,
                              long long ldc, int a_mn_major, int b_mn_major, int epilogue, int block_n, int max_ctas, int flags,
                              cudaStream_t stream) {
@@ -828,6 +978,8 @@ FLB_API int flb_gemm_bf16_ex(const void* A, const void* B, void* C, int M, int N
   DeviceState* st = device_state();
   if (!st) return FLB_ERR_CUDA;
   if (block_n == 0) {
+    if (M <= kFewRows && !a_mn_major && (epilogue == EPI_STORE_BF16 || epilogue == EPI_STORE_F32))
+      return gemm_rows(A, B, C, M, N, K, lda, ldb, ldc, b_mn_major != 0, epilogue, (flags & 2) != 0, st, stream);
     if (M > 256 && N > 256) block_n = 512;
     else block_n = (N >= 256 && (N % 256 == 0 || N > 2048)) ? 256 : 128;
   }

@@ -24,6 +24,7 @@ norm_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __rest
                 const __nv_bfloat16* __restrict__ w, const __nv_bfloat16* __restrict__ b,
                 __nv_bfloat16* __restrict__ res_out, __nv_bfloat16* __restrict__ y, float* __restrict__ rstd_out,
                 float* __restrict__ mean_out, int rows, int cols, float eps, int zero_centered) {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");  // a dependent only reads weights before it waits for this kernel
   __shared__ float scratch[32];
   const int nvec = cols >> 3;
   bf16x8 nx[VPT], nd[VPT];

@@ -17,7 +17,7 @@ from fast_llm_b200.layers.normalization import FixedRMSNormalization, LayerNorma
 from fast_llm_b200.layers.rotary import DefaultRotary, Llama3Rotary, NoRotary, ProportionalRotary, YarnRotary
 from fast_llm_b200.ops import _lib
 
-MAX_ROWS = 16
+MAX_ROWS = 32
 _NORM_KINDS = {RMSNormalization: 1, FixedRMSNormalization: 1, LayerNormalization: 2}
 _ZERO_CENTERED = 4
 
@@ -73,11 +73,8 @@ class DecodePlan:
         self._rotary, self._layers = [], (_Layer * (len(layers) - 2))()
         for out, block in zip(self._layers, layers[1:-1]):
             self._describe(block, out)
-        self._widths = (max(l.heads * l.head_dim for l in self._layers), max((l.heads + 2 * l.kv_heads) * l.head_dim for l in self._layers),
-                        max(l.ffn for l in self._layers))
         self._cache_width = 2 * self._layers[0].kv_heads * self._layers[0].head_dim
         _require(all(2 * l.kv_heads * l.head_dim == self._cache_width for l in self._layers))
-        self._workspaces: dict[tuple, torch.Tensor] = {}
         self._supported = [bool(_lib.get_lib().flb_decode_supported(self._layers, len(self._layers), self._hidden, rows)) for rows in range(MAX_ROWS + 1)]
 
     def _describe(self, block, out: _Layer) -> None:
@@ -115,37 +112,28 @@ class DecodePlan:
     def takes(self, rows: int, new: int, cache) -> bool:
         return new == 1 and cache.length > 0 and rows <= MAX_ROWS and self._supported[rows] and cache.width in (None, self._cache_width)
 
-    def _workspace(self, rows: int, device, stream: int) -> list[torch.Tensor]:
-        """Intermediates of a step, kept per number of rows and stream (a few hundred KB; at most a handful of combinations)."""
-        key = (rows, stream)
-        tensors = self._workspaces.get(key)
-        if tensors is None:
-            if len(self._workspaces) >= 8:
-                self._workspaces.clear()
-            attn, qkv, ffn = self._widths
-            tensors = self._workspaces[key] = [torch.empty(rows, n, dtype=torch.bfloat16, device=device) for n in (self._hidden, self._hidden, qkv, attn, ffn)]
-        return tensors
-
     @torch.no_grad()
     def step(self, tokens: torch.Tensor, cache, device) -> torch.Tensor:
         """tokens [rows, 1]: the next position of every row of `cache`.  Returns logits [rows, vocab] and extends the cache."""
         for stage in self._stages:
             stage.restore_parameters()
         rows, length = tokens.shape[0], cache.length
-        for layer, rotary in zip(self._layers, self._rotary):
-            if rotary is not None:
-                layer.table = rotary.get_table(length + 2, device).data_ptr()
+        # this call's own copy: another thread may step the same model
+        layers = type(self._layers).from_buffer_copy(self._layers)
+        tables = [None if rotary is None else rotary.get_table(length + 2, device) for rotary in self._rotary]
+        for layer, table in zip(layers, tables):
+            layer.table = _lib.ptr(table)
         ids = tokens.reshape(-1).to(device=device, dtype=torch.int64).contiguous()  # a column of a wider tensor stays strided otherwise
         buffer, pads = cache.reserve(length + 1, len(self._layers), self._cache_width, device)
-        stream = _lib.stream_ptr()
-        work = self._workspace(rows, device, stream)
+        lib = _lib.get_lib()
+        workspace = torch.empty(lib.flb_decode_workspace(layers, len(layers), self._hidden, rows), dtype=torch.uint8, device=device)
         logits = torch.empty(rows, self._vocab, dtype=torch.float32, device=device)
         final_w, final_b, final_norm, final_eps = self._final
-        _lib.check(_lib.get_lib().flb_decode_step(
-            self._layers, len(self._layers), ids.data_ptr(), rows, self._embedding, self._embedding_scale, self._hidden, self._vocab, final_w, final_b,
+        _lib.check(lib.flb_decode_step(
+            layers, len(layers), ids.data_ptr(), rows, self._embedding, self._embedding_scale, self._hidden, self._vocab, final_w, final_b,
             final_norm, final_eps, self._head, buffer.data_ptr(), buffer.stride(0), buffer.shape[2], length, pads.data_ptr(),
-            *(t.data_ptr() for t in work), logits.data_ptr(), stream), "flb_decode_step")
-        _lib.count_launch(5 * len(self._layers) + 2)
+            workspace.data_ptr(), logits.data_ptr(), _lib.stream_ptr()), "flb_decode_step")
+        _lib.count_launch(9 * len(layers) + 4)
         cache.length = length + 1
         c = self._head_config
         if c.logits_scale_factor != 1.0:

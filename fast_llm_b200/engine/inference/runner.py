@@ -14,8 +14,9 @@ class KeyValueCache:
     it is a document of its own, as in the packed forward pass).  Parity: the `past_key_values` / `presents` lists of
     `fast_llm/models/gpt/huggingface.py:158-199`.
 
-    Generation steps append to one buffer `[layers, rows, capacity, width]` that grows by doubling, so a step writes its own
-    position instead of copying all earlier ones."""
+    Generation steps append to one buffer `[layers, rows, capacity, width]` with room for more positions (an eighth, at least 256),
+    so a step writes its own position instead of copying all earlier ones.  Where the memory does not have that room, the buffer
+    is exactly as long as asked for."""
 
     def __init__(self, pads: list[int]):
         self.pads = list(pads)  # left padding of every row
@@ -50,12 +51,19 @@ class KeyValueCache:
     def reserve(self, length: int, layers: int, width: int, device) -> tuple[torch.Tensor, torch.Tensor]:
         """(buffer with room for `length` positions of every row, left padding of the rows on the device)."""
         if self._buffer is None or self._buffer.shape[2] < length:
-            buffer = torch.empty(layers, self.rows, -(-2 * length // 64) * 64, width, dtype=torch.bfloat16, device=device)
+            def allocate(capacity):
+                return torch.empty(layers, self.rows, capacity, width, dtype=torch.bfloat16, device=device)
+
+            try:
+                buffer = allocate(-(-(length + max(length // 8, 256)) // 64) * 64)
+            except torch.cuda.OutOfMemoryError:
+                buffer = allocate(length)
             if self._buffer is not None:
                 buffer[:, :, : self.length] = self._buffer[:, :, : self.length]
             else:
                 for i, kv in enumerate(self._layers):
                     buffer[i, :, : self.length] = kv.view(self.rows, self.length, width)
+            buffer[:, :, self.length :] = 0  # masked keys are still multiplied: they have to be finite
             self._buffer, self._layers = buffer, []
         if self._device_pads is None:
             self._device_pads = torch.tensor(self.pads, dtype=torch.int32, device=device)
@@ -95,6 +103,7 @@ class InferenceRunner:
     def __init__(self, model):
         self._model = model
         self._is_setup = False
+        self._plan: tuple | None = None
 
     @property
     def model(self):
@@ -154,13 +163,18 @@ class InferenceRunner:
         blocks = [layer.unwrap() for layer in self._model.base_model.get_layers() if isinstance(layer.unwrap(), DecoderBlock)]
         return bool(blocks) and all(type(block.mixer) is Attention and block.mixer._sdp_dim.size == 1 for block in blocks)
 
-    def _decode_plan(self):
-        """Description of the decoder for the native generation step, None if some part of it has to run layer by layer."""
-        if not hasattr(self, "_plan"):
+    def _decode_plan(self, cache: KeyValueCache):
+        """Description of the decoder for the native generation step, None if some part of it has to run layer by layer.  It
+        holds weight addresses, so every new request (the pass over its prompt) has the decoder described afresh."""
+        if cache.length == 0:
+            self._plan = None
+            return None
+        described = self._plan
+        if described is None:
             from fast_llm_b200.engine.inference.decode import DecodePlan
 
-            self._plan = DecodePlan.build(self._model)
-        return self._plan
+            described = self._plan = (DecodePlan.build(self._model),)
+        return described[0]
 
     @torch.no_grad()
     def forward_rows(self, tokens: torch.Tensor, cache: KeyValueCache, output_hidden_states=None):
@@ -170,7 +184,7 @@ class InferenceRunner:
 
         rows, new = tokens.shape
         assert rows == cache.rows
-        if not output_hidden_states and (plan := self._decode_plan()) is not None and plan.takes(rows, new, cache):
+        if not output_hidden_states and (plan := self._decode_plan(cache)) is not None and plan.takes(rows, new, cache):
             return plan.step(tokens, cache, self._distributed.device), {}
         held = cache.length
         cu_q, cu_k, positions, documents = [0], [0], [], []

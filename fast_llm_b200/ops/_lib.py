@@ -23,7 +23,8 @@ _SIGNATURES = {
     "flb_causal_conv1d_bwd": [_p, _p, _p, _p, _p, _p, _p, _p, _ll, _i, _i, _i, _i, _p],
     "flb_delta_state_scan": [_p, _p, _p, _p, _p, _i, _i, _i, _i, _i, _i, _p],
     "flb_decode_supported": [_p, _i, _i, _i],
-    "flb_decode_step": [_p, _i, _p, _i, _p, _f, _i, _i, _p, _p, _i, _f, _p, _p, _ll, _i, _i] + [_p] * 8,
+    "flb_decode_workspace": [_p, _i, _i, _i],
+    "flb_decode_step": [_p, _i, _p, _i, _p, _f, _i, _i, _p, _p, _i, _f, _p, _p, _ll, _i, _i] + [_p] * 4,
     "flb_delta_max_chunks": [_ll, _i],
     "flb_delta_chunks": [_p, _i, _i, _p, _p, _p],
     "flb_delta_fwd": [_p] * 3 + [_ll] * 3 + [_p] * 2 + [_i] * 6 + [_f] + [_p] * 2 + [_i] * 2 + [_p] * 13,

@@ -852,6 +852,29 @@ def test_delta_rule_kernels(per_channel, tokens, boundaries, heads, key_heads, d
         assert float((a - b).norm()) < 1e-3 * float(b.norm()) + 1e-5 * b.numel() ** 0.5, name
 
 
+@pytest.mark.parametrize("m, n, k, b_mn, dtype", [
+    (1, 8, 8, False, torch.bfloat16),  # less than one tile either way
+    (32, 3072, 2048, False, torch.bfloat16),  # 32-wide tiles, more stages than the ring has
+    (7, 1003, 776, False, torch.float32),  # ragged columns and a ragged last k block
+    (16, 18977, 264, False, torch.float32),  # 64-wide tiles, an odd row stride
+    (5, 200, 8192, True, torch.bfloat16),  # N-major B, the last panel half empty
+    (32, 64, 72, True, torch.bfloat16),
+])
+def test_few_rows_gemm_same_bits(m, n, k, b_mn, dtype):
+    """Up to 32 rows take the narrow tiles: the same products added in the same order as in the wide ones."""
+    from fast_llm_b200.ops.gemm import gemm_raw, matmul_nn, matmul_nt
+
+    torch.manual_seed(1)
+    a = torch.randn(m, k, device="cuda").bfloat16()
+    b = torch.randn((k, n) if b_mn else (n, k), device="cuda").bfloat16()
+    out = (matmul_nn if b_mn else matmul_nt)(a, b, out_dtype=dtype)
+    wide = gemm_raw(a, b, torch.empty(m, n, dtype=dtype, device="cuda"), m, n, k, False, b_mn, 0 if dtype == torch.bfloat16 else 1, block_n=128)
+    assert torch.equal(out, wide)
+    # fp32 sums of k products of order one: k 2^-24 at most; the bf16 result rounds by 2^-9
+    exact = a.double() @ (b if b_mn else b.t()).double()
+    assert float((out.double() - exact).norm() / exact.norm()) < (2**-8 if dtype == torch.bfloat16 else 1e-5)
+
+
 def _decoder(heads, kv_heads, head_size, hidden, ffn, vocab, norm, gated, window, bias):
     import fast_llm_b200.models.auto  # noqa: F401
     from fast_llm_b200.engine.inference.huggingface import HuggingfaceGPTModelForCausalLM
@@ -883,7 +906,7 @@ def _decoder(heads, kv_heads, head_size, hidden, ffn, vocab, norm, gated, window
 
 @pytest.mark.parametrize("rows, prompt, steps, shape", [
     (1, 3, 4, dict(heads=4, kv_heads=2, head_size=64, hidden=256, ffn=512, vocab=512, norm="rms_norm", gated=True, window=0, bias=False)),
-    (9, 70, 3, dict(heads=16, kv_heads=1, head_size=64, hidden=512, ffn=1040, vocab=515, norm="layer_norm", gated=False, window=0, bias=True)),
+    (19, 70, 3, dict(heads=16, kv_heads=1, head_size=64, hidden=512, ffn=1040, vocab=515, norm="layer_norm", gated=False, window=0, bias=True)),
     (16, 130, 3, dict(heads=4, kv_heads=4, head_size=128, hidden=512, ffn=1536, vocab=1000, norm="rms_norm", gated=True, window=33, bias=False)),
     (2, 1100, 2, dict(heads=8, kv_heads=1, head_size=128, hidden=1024, ffn=2048, vocab=1024, norm="rms_norm", gated=True, window=0, bias=False)),
 ])
@@ -895,11 +918,11 @@ def test_native_generation_step(rows, prompt, steps, shape):
     mask = torch.ones(rows, prompt + steps, dtype=torch.int64, device="cuda")
     for row in range(1, rows):
         mask[row, : (row * 7) % max(prompt // 2, 1)] = 0
-    plan = model._inference_runner._decode_plan()
-    assert plan is not None
     with torch.no_grad():
         full = model(input_ids=ids, attention_mask=mask, use_cache=False).logits
         out = model(input_ids=ids[:, :prompt], attention_mask=mask[:, :prompt], use_cache=True)
+        plan = model._inference_runner._decode_plan(out.past_key_values)
+        assert plan is not None
         for step in range(steps):
             assert plan.takes(rows, 1, out.past_key_values)
             out = model(input_ids=ids[:, prompt + step : prompt + step + 1], past_key_values=out.past_key_values, use_cache=True)

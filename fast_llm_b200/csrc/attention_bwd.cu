@@ -67,7 +67,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + C::BARS + 8 * 16);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
   const int kv_head = blockIdx.y;
   const int group = p.heads / p.kv_heads;
   const int doc = blockIdx.x / p.kv_blocks_per_doc;
@@ -111,7 +111,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
   auto pair_q0 = [&](int n) { return (iblk_lo + n % blocks) * BM; };
 
   if (warp == 0) {
-    if (lane == 0) {
+    if (elect_one()) {
       mbar_expect_tx(bar(0), 2 * C::TILE);
       for (int c = 0; c < C::PANELS; ++c) {
         tma_load_3d(sb + C::K + c * PANEL, &tmap_k, bar(0), c * 64, kv_head, k_begin + k0);
@@ -131,7 +131,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
+    if (elect_one()) {
       constexpr uint32_t idesc_kk = make_idesc(128, 128, false, false);  // A K-major, B K-major      (S, dP)
       constexpr uint32_t idesc_mm = make_idesc(128, HD, true, true);    // A MN-major, B MN-major    (dV, dK)
       constexpr uint32_t idesc_km = make_idesc(128, HD, false, true);   // A K-major, B MN-major     (dQ)

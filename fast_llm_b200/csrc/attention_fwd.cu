@@ -75,7 +75,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + SMEM_BARS + 8 * 16);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
   const int head = blockIdx.y;
   const int kv_head = head / (p.heads / p.kv_heads);
   const int doc = blockIdx.x / p.blocks_per_doc;
@@ -116,7 +116,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
   // TMEM columns: S_0 | S_1 | O_0 | O_1
 
   if (warp == 0) {
-    if (lane == 0) {
+    if (elect_one()) {
       // ---- producer
       for (int t = 0; t < num_q; ++t) {
         mbar_expect_tx(bar(t), TILE_BYTES_ATTN);
@@ -139,7 +139,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
+    if (elect_one()) {
       // ---- MMA issuer
       constexpr uint32_t idesc_qk = make_idesc(BM, BN, false, false);
       constexpr uint32_t idesc_pv = make_idesc(BM, D, false, true);
@@ -384,7 +384,7 @@ attn_fwd_kernel_v2(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + C::BARS + 8 * 16);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
   const int head = blockIdx.y;
   const int kv_head = head / (p.heads / p.kv_heads);
   const int doc = blockIdx.x / p.blocks_per_doc;
@@ -424,7 +424,7 @@ attn_fwd_kernel_v2(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
   // TMEM columns: S_0 (P_0 over its first 64) | S_1 (P_1) | O_0 | O_1
 
   if (warp == 0) {
-    if (lane == 0) {
+    if (elect_one()) {
       // ---- producer
       for (int t = 0; t < num_q; ++t) {
         mbar_expect_tx(bar(t), C::TILE);
@@ -447,7 +447,7 @@ attn_fwd_kernel_v2(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
+    if (elect_one()) {
       // ---- MMA issuer
       constexpr uint32_t idesc_qk = make_idesc(BM, BN, false, false);
       constexpr uint32_t idesc_pv = make_idesc(BM, HD, false, true);

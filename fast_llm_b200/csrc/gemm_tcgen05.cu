@@ -70,7 +70,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * C::STAGES + 4);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0);
   const int lane = threadIdx.x & 31;
 
   if (threadIdx.x == 0) {
@@ -106,7 +106,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
 
   if (warp == 0) {
     // ---------------- TMA producer ----------------
-    if (lane == 0) {
+    if (elect_one()) {
       int stage = 0;
       uint32_t phase = 0;
       bool ok = true;
@@ -144,7 +144,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
     }
   } else if (warp == 1) {
     // ---------------- MMA issuer ----------------
-    if (lane == 0) {
+    if (elect_one()) {
       constexpr uint32_t idesc = make_idesc(BLOCK_M, BLOCK_N, A_MN, B_MN);
       int stage = 0;
       uint32_t phase = 0;
@@ -249,7 +249,7 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
   const uint32_t done_bar = bars + 8u * (2 * C::STAGES);
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem_raw + pad + C::BARS + 8 * (2 * C::STAGES + 1));
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
   if (threadIdx.x == 0) {
     for (int s = 0; s < C::STAGES; ++s) {
       mbar_init(full_bar(s), 1);
@@ -271,7 +271,7 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
   const int n0 = blockIdx.x * BLOCK_N, num_kb = (K + BLOCK_K - 1) / BLOCK_K;
 
   if (warp == 1) {
-    if (lane == 0) {
+    if (elect_one()) {
       auto load_b = [&](int kb, int s) {
         mbar_expect_tx(full_bar(s), C::A_BYTES + C::B_BYTES);
         if constexpr (!B_MN) tma_load_2d(base + C::B_OFFSET + s * C::B_BYTES, &tmap_b, full_bar(s), kb * BLOCK_K, n0);
@@ -296,7 +296,7 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
       }
     }
   } else if (warp == 2) {
-    if (lane == 0) {
+    if (elect_one()) {
       constexpr uint32_t idesc = make_idesc(BLOCK_M, BLOCK_N, false, B_MN);
       bool ok = true;
       for (int kb = 0; kb < num_kb; ++kb) {
@@ -514,7 +514,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * C::STAGES + 4);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0);
   const int lane = threadIdx.x & 31;
   const uint32_t cta_rank = cluster_ctarank();
   const bool leader = cta_rank == 0;
@@ -558,7 +558,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
 
   if (warp == 0) {
     // ---------------- TMA producer (one per CTA; transaction bytes are counted on the leader's barrier) ----------------
-    if (lane == 0) {
+    if (elect_one()) {
       int stage = 0;
       uint32_t phase = 0;
       bool ok = true;
@@ -609,7 +609,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
     }
   } else if (warp == 1) {
     // ---------------- MMA issuer (leader CTA only) ----------------
-    if (lane == 0 && leader) {
+    if (leader && elect_one()) {
       constexpr uint32_t idesc = make_idesc(C::TILE_M, C::TILE_N, A_MN, B_MN);
       int stage = 0;
       uint32_t phase = 0;

@@ -5,7 +5,8 @@
 // one after another on the same numbers in the same order (the same logits, bit for bit), with three differences: the new keys and
 // values are appended to one cache buffer instead of copying all earlier ones, the residual add after the MLP rides in the next
 // block's norm, and the GEMMs (gemm_rows_kernel) start reading their weights while the kernel ahead of them runs.
-// 8 blocks of 2048 / 8192, 24 steps: see the comment at flb_decode_step.
+// 8 blocks of 2048 / 8192, a prompt and 24 steps: one row after 100 positions 92 -> 18.5 ms, 8 rows after 512 95 -> 22 ms; a step is 0.6 ms
+// of kernels one after another, half of it the GEMMs of the MLP.
 #include "common.cuh"
 
 FLB_API int flb_norm_fwd(const void* x, const void* delta, const void* w, const void* b, void* res_out, void* y, float* rstd, float* mean, int rows,

@@ -221,25 +221,26 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
 // Few rows (up to 32, a generation step): one narrow tile per CTA
 // ------------------------------------------------------------------------------------------------
 // Bounded by the weights' trip from HBM: 256-wide tiles leave a 3072-wide projection on 12 SMs with 128 KB in flight in all.  Tiles
-// of 32 columns (64 where B is N-major or there are enough of them for the chip) and deep rings put every SM to work.  Of the 128
+// of 32 columns (64 where B is N-major or there are enough of them for the chip) and deep rings put the SMs to work.  Of the 128
 // rows of A that the MMA reads only 32 are copied: the rest is whatever shared memory holds (later stages, B), its accumulator
 // rows are never read.  The MMAs of an output element are those of the wide tiles in the same order, so the results are the same
-// bits.  8 blocks of 2048 / 8192, 24 steps of one row after a prompt of 100 and of 8 rows after 512: see flb_decode_step.
+// bits.  One row: [2048] x 3072 7.8 us, x 16384 16.8 us, x 32000 29.3 us; [8192] x 2048 (N-major) 20.4 us, where the chain of 512
+// dependent MMAs takes 15 whatever the tile (32-wide panels: 21.7; 24 stages: 3072 columns in 9.0).
 constexpr int kFewRows = 32;
-template <int BLOCK_N>
+template <int BLOCK_N, int STAGE_COUNT>
 struct RowsCfg {
   static constexpr int A_BYTES = kFewRows * BLOCK_K * 2, B_BYTES = BLOCK_N * BLOCK_K * 2;
-  static constexpr int STAGES = BLOCK_N == 32 ? 12 : 16;
+  static constexpr int STAGES = STAGE_COUNT;
   static constexpr int B_OFFSET = STAGES * A_BYTES, BARS = B_OFFSET + STAGES * B_BYTES;
   static constexpr int SMEM_BYTES = BARS + 512 + 1024;
   static_assert((STAGES - 1) * A_BYTES + BLOCK_M * BLOCK_K * 2 <= BARS, "the MMA's 128 rows stay inside the allocation");
 };
 
-template <int BLOCK_N, bool B_MN, int EPI>
+template <int BLOCK_N, int STAGE_COUNT, bool B_MN, int EPI>
 __global__ void __launch_bounds__(96)
 gemm_rows_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b, void* __restrict__ Cv, int M, int N, int K,
                  long long ldc, int* __restrict__ err_word) {
-  using C = RowsCfg<BLOCK_N>;
+  using C = RowsCfg<BLOCK_N, STAGE_COUNT>;
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw_addr = smem_u32(smem_raw);
   const uint32_t pad = (1024u - (raw_addr & 1023u)) & 1023u;
@@ -868,10 +869,10 @@ int launch(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& tc, 
   return FLB_OK;
 }
 
-template <int BLOCK_N, bool B_MN, int EPI>
+template <int BLOCK_N, int STAGE_COUNT, bool B_MN, int EPI>
 int launch_rows(const CUtensorMap& ta, const CUtensorMap& tb, void* C, int M, int N, int K, long long ldc, bool overlap, DeviceState* st, cudaStream_t stream) {
-  using Cf = RowsCfg<BLOCK_N>;
-  auto kern = gemm_rows_kernel<BLOCK_N, B_MN, EPI>;
+  using Cf = RowsCfg<BLOCK_N, STAGE_COUNT>;
+  auto kern = gemm_rows_kernel<BLOCK_N, STAGE_COUNT, B_MN, EPI>;
   static const cudaError_t ready = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Cf::SMEM_BYTES);
   if (ready != cudaSuccess) return flb_record_cuda_error(ready);
   cudaLaunchConfig_t config{};
@@ -891,18 +892,19 @@ int launch_rows(const CUtensorMap& ta, const CUtensorMap& tb, void* C, int M, in
 // Up to 32 rows: see gemm_rows_kernel.
 int gemm_rows(const void* A, const void* B, void* C, int M, int N, int K, long long lda, long long ldb, long long ldc, bool b_mn, int epilogue,
               bool overlap, DeviceState* st, cudaStream_t stream) {
-  // 32-wide tiles until two waves of 64-wide ones fill the chip; an N-major panel is 64 columns
-  const bool narrow = !b_mn && N <= 2 * 64 * st->num_sms;
+  // 64-wide tiles (two CTAs an SM) where they fill the chip, 32-wide ones below: 16384 columns 22.7 -> 16.8 us, 32000 34.5 -> 29.3 us.
+  // An N-major panel is 64 columns; few CTAs, so each takes a deep ring.
+  const bool narrow = !b_mn && N < 64 * st->num_sms;
   CUtensorMap ta, tb;
   if (!make_tmap(&ta, A, (uint64_t)K, (uint64_t)M, (uint64_t)lda, BLOCK_K, kFewRows)) return FLB_ERR_TMA;
   if (!(b_mn ? make_tmap(&tb, B, (uint64_t)N, (uint64_t)K, (uint64_t)ldb, 64, BLOCK_K)
              : make_tmap(&tb, B, (uint64_t)K, (uint64_t)N, (uint64_t)ldb, BLOCK_K, narrow ? 32 : 64))) return FLB_ERR_TMA;
-#define FLB_ROWS(BN, MN)                                                                                                             \
-  return epilogue == EPI_STORE_F32 ? launch_rows<BN, MN, EPI_STORE_F32>(ta, tb, C, M, N, K, ldc, overlap, st, stream)               \
-                                   : launch_rows<BN, MN, EPI_STORE_BF16>(ta, tb, C, M, N, K, ldc, overlap, st, stream)
-  if (b_mn) FLB_ROWS(64, true);
-  if (narrow) FLB_ROWS(32, false);
-  FLB_ROWS(64, false);
+#define FLB_ROWS(BN, STAGES, MN)                                                                                                     \
+  return epilogue == EPI_STORE_F32 ? launch_rows<BN, STAGES, MN, EPI_STORE_F32>(ta, tb, C, M, N, K, ldc, overlap, st, stream)       \
+                                   : launch_rows<BN, STAGES, MN, EPI_STORE_BF16>(ta, tb, C, M, N, K, ldc, overlap, st, stream)
+  if (b_mn) FLB_ROWS(64, 16, true);
+  if (narrow) FLB_ROWS(32, 12, false);
+  FLB_ROWS(64, 8, false);
 #undef FLB_ROWS
 }
 

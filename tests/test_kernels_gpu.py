@@ -859,6 +859,8 @@ def test_delta_rule_kernels(per_channel, tokens, boundaries, heads, key_heads, d
     (16, 18977, 264, False, torch.float32),  # 64-wide tiles, an odd row stride
     (5, 200, 8192, True, torch.bfloat16),  # N-major B, the last panel half empty
     (32, 64, 72, True, torch.bfloat16),
+    (3, 6000, 512, False, torch.bfloat16),  # more 32-wide tiles than SMs
+    (4, 9480, 200, True, torch.float32),  # more panels than SMs
 ])
 def test_few_rows_gemm_same_bits(m, n, k, b_mn, dtype):
     """Up to 32 rows take the narrow tiles: the same products added in the same order as in the wide ones."""
